@@ -16,11 +16,12 @@
 //   bitrev_cols: tile (column, mid) holds words (hi << (L-5)) | (mid << 5) | lo
 //     for hi, lo < 32; word (hi, mid, lo) goes to (rev5(lo), rev(mid), rev5(hi));
 //     tiles mid and rev(mid) swap, so the permutation also runs in place.
-//   transpose: tile (32 columns) x (32 consecutive rows); each row of the tile
-//     becomes 32 consecutive words of one output row.
+//   transpose: tiles of columns x consecutive rows; each row of the tile
+//     becomes consecutive words of one output row.
 #include <algorithm>
 
 #include "context.hpp"
+#include "tma_launch.cuh"
 
 namespace sfntt {
 namespace {
@@ -115,6 +116,111 @@ __global__ void __launch_bounds__(kWideThreads) bitrev_cols64_kernel(const uint3
   }
 }
 
+// Row-major rows of up to 256 columns (log_n >= 5, 16-byte aligned buffers):
+// tiles of every column x 32 kr rows, about 32 KiB.  TMA brings a tile in as
+// 128-byte pieces, line = piece * batch + column, with the 128-byte swizzle; a
+// lane then takes 4 consecutive rows of its column with one 128-bit load (lanes
+// on consecutive columns: the swizzle spreads 8 of them over all banks) and
+// writes them as four words of the row-major tile.  In row order that tile is
+// one contiguous run of the output and leaves as one bulk copy, so a row of 400
+// bytes costs no partial sectors; bit-reversed rows leave as one copy each
+// (rows of whole 16-byte units) or by coalesced stores.  Bound by HBM (8 bytes
+// per word; the reads are 128-byte runs megabytes apart); two input tiles per
+// CTA keep the next load in flight.  Row order 2^19 x 100: 125 -> 70 us (6.0
+// TB/s) against the 32 x 32 tiles, 2^21 x 256: 858 -> 756 us against the
+// 128-column tiles, 2^20 x 7: 58 -> 25 us; bit-reversed 2^19 x 100: 144 -> 107
+// us, 2^21 x 256: 873 -> 740 us.
+constexpr uint32_t kRowsThreads = 256;
+constexpr uint32_t kRowsMaxLines = 256;
+struct RowsArgs {
+  uint32_t* out;
+  uint32_t log_n, batch;
+  uint32_t lk;     // log2 of the 32-row pieces per tile
+  uint32_t tiles;
+  uint32_t bitrev;
+  int* err;
+};
+
+__global__ void __launch_bounds__(kRowsThreads) transpose_tma_kernel(const __grid_constant__ CUtensorMap map_in,
+                                                                     RowsArgs a) {
+  extern __shared__ __align__(1024) uint32_t smem_rows[];
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t nb = a.batch, words = nb << (a.lk + 5);
+  const uint32_t in_words = (words + 255u) & ~255u;  // 1024-byte aligned tiles (swizzle)
+  uint32_t* ot = smem_rows + 2 * in_words;           // the row-major tile
+  uint64_t* bar = reinterpret_cast<uint64_t*>(ot + in_words);
+  uint32_t t = blockIdx.x;
+  if (t >= a.tiles) return;
+  auto load = [&](uint32_t tile, uint32_t buf) {
+    tma::mbar_expect_tx(&bar[buf], words * 4u);
+    tma::load_3d(smem_rows + buf * in_words, &map_in, 0, 0, (int32_t)(tile << a.lk), &bar[buf]);
+  };
+  if (tid == 0) {
+    tma::prefetch_map(&map_in);
+    tma::mbar_init(&bar[0], 1);
+    tma::mbar_init(&bar[1], 1);
+    tma::fence_mbar_init();
+  }
+  __syncthreads();
+  if (tid == 0) load(t, 0);
+  const uint32_t cgroups = (nb + 31u) >> 5;
+  const uint32_t units = (cgroups << a.lk) * 8u;  // (piece, column group, 4-row chunk)
+  for (uint32_t it = 0; t < a.tiles; t += gridDim.x, ++it) {
+    const uint32_t buf = it & 1u;
+    const uint32_t* it_in = smem_rows + buf * in_words;
+    const uint32_t tn = t + gridDim.x;
+    if (tid == 0 && tn < a.tiles) load(tn, buf ^ 1u);  // that buffer's readers passed the last barrier
+    if (warp == 0) tma::wait_reads();                  // the previous tile's stores have read `ot`
+    const bool ok = tma::mbar_wait(&bar[buf], (it >> 1) & 1u, kWaitNs);
+    __syncthreads();
+    for (uint32_t u = warp; u < units; u += kRowsThreads / 32) {
+      const uint32_t j = u & 7u, pg = u >> 3;
+      const uint32_t piece = pg / cgroups, col = ((pg - piece * cgroups) << 5) + lane;
+      if (col < nb) {
+        const uint32_t line = piece * nb + col;
+        const uint4 q = *reinterpret_cast<const uint4*>(it_in + line * 32u + ((j ^ (line & 7u)) << 2));
+        uint32_t* d = ot + (piece * 32u + j * 4u) * nb + col;
+        d[0] = q.x;
+        d[nb] = q.y;
+        d[2 * nb] = q.z;
+        d[3 * nb] = q.w;
+      }
+    }
+    tma::fence_proxy_async();
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0) {
+        atomicExch(a.err, 1);
+        if (tn < a.tiles) tma::mbar_wait(&bar[buf ^ 1u], ((it + 1) >> 1) & 1u, kWaitNs);
+      }
+      if (warp == 0) tma::wait_all();
+      return;
+    }
+    const uint32_t r0 = t << (5 + a.lk);
+    if (!a.bitrev) {
+      if (tid == 0) {
+        tma::store_bulk(a.out + (uint64_t)r0 * nb, ot, words * 4u);
+        tma::commit();
+      }
+      continue;
+    }
+    // row i of the tile goes to output row bitrev(r0 + i) = bitrev(r0) + (bitrev(i) << ..)
+    const uint32_t R0 = rev_bits(r0, a.log_n), sh = a.log_n - 5 - a.lk;
+    if ((nb & 3u) == 0) {
+      if (warp == 0) {
+        for (uint32_t i = lane; i < (32u << a.lk); i += 32)
+          tma::store_bulk(a.out + (uint64_t)(R0 + (rev_bits(i, 5 + a.lk) << sh)) * nb, ot + i * nb, nb * 4u);
+        tma::commit();
+      }
+    } else {
+      for (uint32_t i = warp; i < (32u << a.lk); i += kRowsThreads / 32) {
+        uint32_t* d = a.out + (uint64_t)(R0 + (rev_bits(i, 5 + a.lk) << sh)) * nb;
+        for (uint32_t c = lane; c < nb; c += 32) d[c] = ot[i * nb + c];
+      }
+    }
+  }
+  if (warp == 0) tma::wait_all();
+}
+
 // Row-major on 128-column x 32-row tiles (log_n >= 5, batch >= 128): 128-byte
 // reads (32 rows of one column) and 512-byte writes (128 columns of one row),
 // so a tile's output is 32 runs of 512 bytes, one per output row.  Tile word
@@ -163,7 +269,8 @@ __global__ void __launch_bounds__(kWideThreads) transpose_wide_kernel(const uint
   }
 }
 
-// log_n >= 5.  Tiles: ceil(batch / 32) column blocks x (n / 32) row blocks.
+// Row-major rows of small batches and of buffers without 16-byte alignment:
+// 32 x 32 tiles (log_n >= 5).  Tiles: ceil(batch / 32) column blocks x (n / 32) row blocks.
 __global__ void __launch_bounds__(kLayoutThreads) transpose_kernel(const uint32_t* __restrict__ in,
                                                                    uint32_t* __restrict__ out, uint32_t log_n,
                                                                    uint32_t batch, uint32_t cblocks, uint64_t tiles,
@@ -269,6 +376,33 @@ Status layout_dev(sfntt_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t lo
     if (!same) SFNTT_CU(cudaMemcpyAsync(out, in, total * 4, cudaMemcpyDeviceToDevice, s));
     return {};
   }
+  const char* name = natural ? "layout_transpose_bitrev" : "layout_transpose";
+  // The TMA tiles pay from 2^22 words on (below, the launch and the first
+  // tile's latency are the cost: 2^15 x 128 9.3 us here, 10.0 us there).  Above
+  // 256 columns a tile no longer holds whole rows (2^19 x 301 in column blocks:
+  // 333 us against 283 us), and bit-reversed rows of few columns are many small
+  // copies (2^20 x 64: 164 us against 137 us; 2^18 x 75: 42 us against 48 us).
+  if (total >= (1ull << 22) && batch <= kRowsMaxLines && (!natural || batch >= 72) && log_n >= 5 && aligned16(in) &&
+      aligned16(out)) {
+    RowsArgs ra{};
+    while (ra.lk < log_n - 5 && (batch << (ra.lk + 1)) <= kRowsMaxLines) ++ra.lk;
+    ra.out = out; ra.log_n = log_n; ra.batch = batch; ra.bitrev = natural ? 1u : 0u;
+    ra.tiles = 1u << (log_n - 5 - ra.lk);
+    ra.err = ctx->err.as<int>();
+    CUtensorMap map;
+    const cuuint64_t dims[3] = {32, batch, n / 32}, strides[2] = {n * 4, 128};
+    const cuuint32_t box[3] = {32, batch, 1u << ra.lk};
+    SFNTT_TRY(tensor_map_encode(&map, in, 3, dims, strides, box, true));
+    auto smem_of = [](uint32_t lines) { return (int)(3 * ((lines * 128 + 1023) & ~1023u)) + 16 + 1024; };
+    const int smem = smem_of(batch << ra.lk);
+    static std::atomic<uint64_t> smem_done{0};
+    SFNTT_TRY(smem_limit_once(transpose_tma_kernel, smem_of(kRowsMaxLines), ctx->device, smem_done));
+    const uint32_t per_sm = std::min<uint32_t>(8, 232448u / ((uint32_t)smem + 1024));
+    const uint32_t grid = std::min<uint32_t>(ra.tiles, (uint32_t)ctx->sm_count * per_sm);
+    launch_begin(ctx, s);
+    transpose_tma_kernel<<<grid, kRowsThreads, smem, s>>>(map, ra);
+    return launch_check(ctx, name, s, total * 8);
+  }
   launch_begin(ctx, s);
   if (log_n >= 5 && batch >= kWideCols) {
     const uint32_t cblocks = (batch + kWideCols - 1) / kWideCols;
@@ -284,7 +418,7 @@ Status layout_dev(sfntt_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t lo
     const uint64_t tiles = (uint64_t)cblocks << (log_n - 5);
     transpose_kernel<<<grid_for(ctx, tiles), kLayoutThreads, 0, s>>>(in, out, log_n, batch, cblocks, tiles,
                                                                       natural ? 1 : 0);
-    return launch_check(ctx, natural ? "layout_transpose_bitrev" : "layout_transpose", s, total * 8);
+    return launch_check(ctx, name, s, total * 8);
   }
   layout_words_kernel<<<grid_for(ctx, (total + 255) / 256), 256, 0, s>>>(in, out, log_n, batch, total, flags);
   return launch_check(ctx, "layout_words", s, total * 8);

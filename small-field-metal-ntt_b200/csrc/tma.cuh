@@ -93,6 +93,14 @@ __device__ __forceinline__ void store_5d(const CUtensorMap* map, int32_t c0, int
                : "memory");
 }
 
+// Untiled store of `bytes` (a multiple of 16) from shared to global memory, both 16-byte aligned.
+__device__ __forceinline__ void store_bulk(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
+                   static_cast<uint64_t>(__cvta_generic_to_global(dst))),
+               "r"(smem_addr(src)), "r"(bytes)
+               : "memory");
+}
+
 __device__ __forceinline__ void commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 
 // All committed stores have finished reading shared memory.
