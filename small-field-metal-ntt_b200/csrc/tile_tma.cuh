@@ -194,13 +194,19 @@ struct TPass {
     }
   }
 
+  // 128-byte rows of spanning columns (one long column of batch << log_n words).
+  __device__ static __forceinline__ int32_t span_rows(const TmaArgs& a) {
+    return (KD == Kind::C && a.spans) ? (int32_t)(((uint64_t)a.batch << a.log_n) >> 5) : INT32_MAX;
+  }
+
   __device__ static __forceinline__ void tma_load(const CUtensorMap* m, const Geo& g, uint32_t* dst, uint64_t* bar) {
     if constexpr (KD == Kind::C) c_load(m, g.c1, g.c2, dst, bar, true);
     else tma::load_5d(dst, m, 0, g.s1, 0, g.s3, g.s4, bar);
   }
 
-  __device__ static __forceinline__ void tma_store(const CUtensorMap* m, const Geo& g, const uint32_t* src) {
-    if constexpr (KD == Kind::C) c_store(m, g.c1, g.c2, src, true);
+  __device__ static __forceinline__ void tma_store(const CUtensorMap* m, const Geo& g, const uint32_t* src,
+                                                   int32_t rows = INT32_MAX) {
+    if constexpr (KD == Kind::C) c_store(m, g.c1, g.c2, src, true, rows);
     else tma::store_5d(m, 0, g.s1, 0, g.s3, g.s4, src);
   }
 
@@ -217,11 +223,15 @@ struct TPass {
       tma::load_3d(dst, m, 0, row, col, bar);
     }
   }
+  // `rows`: rows of the column (the last tile of spanning columns may end past
+  // them: loads fill zeros there and stores clip; a copy that would start past
+  // the end is not issued as a store).
   __device__ static __forceinline__ void c_store(const CUtensorMap* m, int32_t row, int32_t col, const uint32_t* src,
-                                                 bool whole) {
+                                                 bool whole, int32_t rows = INT32_MAX) {
     if constexpr (kRowPerm) {
       tma::store_5d(m, 0, 0, row >> 3, 0, col, src);
-      if (whole) tma::store_5d(m, 0, 0, (row >> 3) + (int32_t)(TWORDS / 512), 0, col, src + TWORDS / 2);
+      if (whole && row + (int32_t)(TWORDS / 64) < rows)
+        tma::store_5d(m, 0, 0, (row >> 3) + (int32_t)(TWORDS / 512), 0, col, src + TWORDS / 2);
     } else {
       tma::store_3d(m, 0, row, col, src);
     }
@@ -841,6 +851,7 @@ struct TPass {
     uint32_t t = blockIdx.x;
     const uint32_t t_end = a.ntiles, t_step = gridDim.x;
     if (t >= t_end) return;
+    const int32_t rows = span_rows(a);
     if constexpr (kStaged) stage_twiddles(tws, a.tw, tid);
     if (leader) {
       tma::prefetch_map(min);
@@ -895,7 +906,7 @@ struct TPass {
         }
         return;
       }
-      if (leader) {
+      if (leader && g.c1 + hrow < rows) {
         c_store(mout, g.c1 + hrow, g.c2, cur, false);
         tma::commit();
       }
@@ -1001,7 +1012,7 @@ struct TPass {
         return;
       }
       if (tid == 0) {
-        tma_store(mout, g, cur);
+        tma_store(mout, g, cur, span_rows(a));
         tma::commit();
       }
     }

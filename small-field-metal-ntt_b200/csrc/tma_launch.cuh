@@ -39,15 +39,22 @@ Status tensor_map_encode(CUtensorMap* map, const void* base, uint32_t rank, cons
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Can a pass of this shape run on the TMA engine?  Contiguous passes over
-// columns shorter than a tile need dense columns (stride n) whose batch fills
-// whole tiles.
+// columns shorter than a tile need dense columns (stride n) of whole 128-byte
+// rows.  A batch that does not fill its last tile takes the engine from 2^18
+// words on (n = 2^12: from one tile): the copies fill and clip what lies past
+// the end.  Below that the one-group-per-CTA passes of the first engine are
+// quicker (BabyBear 2^9 x 41 forward 3.7 against 4.2 us, x 333 4.0 against 4.8
+// us; but x 20001 49.0 against 21.3 us, 2^8 x 4001 9.1 against 4.5 us, 2^12 x 3
+// 7.6 against 5.9 us).
 inline bool tma_pass_ok(const TmaRequest& r) {
   if (!aligned16(r.in) || !aligned16(r.out) || (r.in_stride & 3) || (r.out_stride & 3)) return false;
   const uint64_t n = 1ull << r.log_n;
   if (r.contiguous) {
     if (r.P < 5 || r.P > 14 || r.lo != 0) return false;
     if (n >= kTileWords) return true;
-    return r.in_stride == n && r.out_stride == n && ((uint64_t)r.batch * n) % kTileWords == 0;
+    const uint64_t words = (uint64_t)r.batch * n;
+    return n >= 32 && r.in_stride == n && r.out_stride == n &&
+           (words % kTileWords == 0 || words >= (r.log_n >= 12 ? (uint64_t)kTileWords : 1ull << 18));
   }
   return r.P >= 1 && r.P <= 8 && r.lo >= 5 && r.lo + r.P <= r.log_n;
 }
@@ -121,7 +128,7 @@ Status launch_tma_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
     a.log_tpc = a.spans ? 0u : r.log_n - T::CB;
     // every M31 table with n >= 2^13 carries its first-round copy from entry n on
     if constexpr (T::kRound0Copy) a.tw0 = a.spans ? nullptr : r.tw + n;
-    a.ntiles = (uint32_t)(((uint64_t)r.batch * n) >> T::CB);
+    a.ntiles = (uint32_t)(((uint64_t)r.batch * n + T::TWORDS - 1) >> T::CB);
   } else {
     const uint64_t hb = n >> (r.lo + P);
     SFNTT_TRY(encode_s_map(&min, r.in, r.lo, P, hb, 1ull << (r.lo + P), r.in_stride, r.batch));
