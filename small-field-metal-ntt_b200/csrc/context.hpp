@@ -213,6 +213,15 @@ Status ntt_dev_oop(sfntt_ctx* ctx, int field, bool inverse, const uint32_t* d_in
 // Coset LDE over BabyBear or KoalaBear (lde.cu).
 Status monty_lde_dev(sfntt_ctx* ctx, int field, const uint32_t* d_in, uint32_t* d_out, uint32_t log_n,
                      uint32_t batch, uint32_t added_bits, uint32_t shift_monty, int mode, cudaStream_t stream);
+// The coset LDE / blow-up of 2^5 .. 2^14-point columns in one launch
+// (lde_small.cu).  mul: BabyBear / KoalaBear multipliers (kind 0, from 2^13
+// points on kind 2); scale_w: M31's n^-1.  The input may lie in the output
+// columns only as in == out.
+bool lde_small_fits(const sfntt_ctx* ctx, const uint32_t* in, const uint32_t* out, uint64_t in_stride, uint32_t log_n,
+                    uint32_t batch, uint32_t added_bits);
+Status lde_small_dev(sfntt_ctx* ctx, int field, const uint32_t* in, uint64_t in_stride, uint32_t* out, uint32_t log_n,
+                     uint32_t batch, uint32_t added_bits, const uint2* tw_inv, const uint2* tw_fwd, const uint2* mul,
+                     uint32_t scale_w, cudaStream_t stream);
 // canonic = false: the reference-network composition inverse(odds(log_n)) ->
 // zero-pad -> forward(odds(log_n + added)); true: the canonic-coset circle LDE
 // (same network, canonic circle-FFT twiddles).

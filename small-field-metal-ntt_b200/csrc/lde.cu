@@ -13,6 +13,8 @@
 //       reduces to "copy, and copy times twiddle"), then forward layers
 //       [lo, log_n) of block q, stored to output rows [q n, (q+1) n)
 //   F3  forward layers [0, lo) of the n_ext-point network, in place
+// Columns of 2^5 .. 2^13 points (2^14 in small batches) run all three in one
+// launch, one CTA per column (lde_small.cu).
 // Every HBM byte of the input is read once and every output byte is written
 // twice (X and F3), against the reference's separate iDFT / normalize+pad+
 // shift / DFT passes.
@@ -308,9 +310,11 @@ Status monty_lde_rows(sfntt_ctx* ctx, const uint32_t* d_in, uint64_t in_stride, 
     const uint2 *tw_inv = nullptr, *tw_fwd = nullptr, *mul = nullptr;
     SFNTT_TRY(monty_twiddles(ctx, field, true, log_n, s, &tw_inv));
     SFNTT_TRY(monty_twiddles(ctx, field, false, log_ext, s, &tw_fwd));
-    const bool tma_ok = !ctx->no_tma && log_n >= 13 && aligned16(d_in) && aligned16(d_out);
-    // the TMA expansion reads its multipliers in tile order (kind 2)
-    SFNTT_TRY(monty_lde_table(ctx, field, log_n, added_bits, shift_monty, tma_ok ? 2 : 0, s, &mul));
+    const bool small = lde_small_fits(ctx, d_in, d_out, in_stride, log_n, batch, added_bits);
+    const bool tma_ok = !small && !ctx->no_tma && log_n >= 13 && aligned16(d_in) && aligned16(d_out);
+    // the TMA expansion reads its multipliers in tile order (kind 2), and so do
+    // the short columns of the sizes that either route may take
+    SFNTT_TRY(monty_lde_table(ctx, field, log_n, added_bits, shift_monty, tma_ok || (small && log_n >= 13) ? 2 : 0, s, &mul));
     if (tma_ok) {
       // I1: inverse layers [0, lo) into the output buffer, ending with the
       // four-step pre-twist of the expand's sub-iDFT; X: the persistent TMA
@@ -340,6 +344,8 @@ Status monty_lde_rows(sfntt_ctx* ctx, const uint32_t* d_in, uint64_t in_stride, 
                            mask));
       return {};
     }
+    if (small)
+      return lde_small_dev(ctx, field, d_in, in_stride, d_out, log_n, batch, added_bits, tw_inv, tw_fwd, mul, 0u, s);
     const uint32_t lo = log_n <= 12 ? 0u : (log_n + 1) / 2;
     const int P = (int)(log_n - lo);
     if (lo > 0) {  // I1: inverse layers [0, lo) into the output buffer
@@ -436,6 +442,9 @@ Status m31_lde_dev(sfntt_ctx* ctx, const uint32_t* d_in, uint32_t* d_out, uint32
     SFNTT_TRY(twiddles(true, log_n, &tw_inv));
     SFNTT_TRY(twiddles(false, log_ext, &tw_fwd));
   }
+  if (lde_small_fits(ctx, d_in, d_out, n, log_n, batch, added_bits))
+    return lde_small_dev(ctx, SFNTT_M31, d_in, n, d_out, log_n, batch, added_bits, tw_inv, tw_fwd, nullptr,
+                         inv_n_of(SFNTT_M31, log_n), s);
   if (!ctx->no_tma && log_n >= 13 && added_bits <= 4 && aligned16(d_in) && aligned16(d_out)) {
     // I1: inverse layers [0, lo) into the output columns; X: inverse layers
     // [lo, log_n), n^-1, and per output block forward layers [lo, log_n) of

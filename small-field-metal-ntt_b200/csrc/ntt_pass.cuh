@@ -85,6 +85,9 @@ __host__ __device__ constexpr int filler_hint(int k, int i) {
   if (KD != Kind::C || R != 4 || i != 0) return -1;
   if (P == 14 && LT == 0) return k == 2 ? 11 : k == 3 ? 7 : -1;
   if (P == 11 && LT == 2) return k == 2 ? 11 : -1;
+  // 2^11-word tiles of short columns (lde_small.cu): round 0 owns tile bits 0..3
+  // whatever its layers, so its threads read and write 16 consecutive words
+  if (P + LT == 11 && Plan<P, R>::r(0) == 3) return k == 0 ? 3 : -1;
   return -1;
 }
 

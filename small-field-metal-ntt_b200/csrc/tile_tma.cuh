@@ -104,8 +104,11 @@ struct TileCoord {
 // per-position twiddles): the caller has staged the twiddles of the tile's
 // 32-position chunk in shared memory (see lchunk_entry), so every twiddle is a
 // shared-memory load instead of an L2 one.
+//
+// TBX (Kind::C): tiles of 2^TBX words holding whole columns of 2^P points, for
+// kernels that run the rounds on tiles of their own (0: the engine's tiles).
 template <class F, bool DESC, Kind KD, int P, bool PLAIN = false, bool TW = false, bool LSTAGE = false,
-          bool HALVES = false>
+          bool HALVES = false, int TBX = 0>
 struct TPass {
   // LSTAGE: each CTA takes a contiguous range of tiles ordered so that it
   // stays on one set of positions across the columns, and stages that set's
@@ -119,7 +122,8 @@ struct TPass {
                 "position staging: BabyBear 8-layer strided or M31 contiguous tiles");
   // Tile bits: 2^13-word tiles, except the 14-layer contiguous pass, whose
   // tile is one 2^14-point group (64 KiB, 1024 threads, one CTA per SM).
-  static constexpr int TB = (KD == Kind::C && P > kTileBits) ? P : kTileBits;
+  static_assert(TBX == 0 || (KD == Kind::C && TBX >= P && !LSTAGE && !HALVES && !TW), "own tile size: whole columns");
+  static constexpr int TB = TBX ? TBX : (KD == Kind::C && P > kTileBits) ? P : kTileBits;
   static constexpr int LT = (KD == Kind::C) ? (TB - P) : 5;
   static constexpr int CB = P + LT;
   static constexpr int R = 4;
@@ -313,6 +317,11 @@ struct TPass {
     for (int i = 0; i < C; ++i) tv[AT + i] = make_uint2(w[i] >> 1, w[i]);
   }
 
+  // Tile bits that are positions in a column (the rest select the column).
+  __device__ static __forceinline__ uint32_t col_mask(const TmaArgs& a) {
+    return (TBX ? (1u << P) : (1u << a.log_n)) - 1u;
+  }
+
   // ---- twiddles: per-layer base pointer + compile-time offset per slot ----
   template <int k>
   __device__ static __forceinline__ uint2 twiddle(const TmaArgs& a, const uint2* tws, const Geo& g, uint32_t ct, int m,
@@ -345,7 +354,7 @@ struct TPass {
       const uint32_t n = 1u << a.log_n;
       const uint2* base = a.tw + (n - (n >> L));
       if constexpr (KD == Kind::C) {  // tile bits above log n select the column (spanning tiles)
-        return __ldg(base + ((g.pos_base >> (L + 1)) + ((ct & (n - 1u)) >> (L + 1)) + ((cm & (n - 1u)) >> (L + 1))));
+        return __ldg(base + ((g.pos_base >> (L + 1)) + ((ct & col_mask(a)) >> (L + 1)) + ((cm & col_mask(a)) >> (L + 1))));
       } else {
         return __ldg(base + ((g.hb << (P - beta - 1)) + ((ct >> 5) >> (beta + 1)) + ((cm >> 5) >> (beta + 1))));
       }
@@ -413,7 +422,7 @@ struct TPass {
           }
           if (!copied) {
             const uint2* base = a.tw + (n - (n >> L));
-            if constexpr (KD == Kind::C) base += (g.pos_base >> (L + 1)) + ((ct & (n - 1u)) >> (L + 1));
+            if constexpr (KD == Kind::C) base += (g.pos_base >> (L + 1)) + ((ct & col_mask(a)) >> (L + 1));
             else base += (g.hb << (P - beta - 1)) + ((ct >> 5) >> (beta + 1));
             if (j == r - 1) {
               tv[0] = __ldg(base);
