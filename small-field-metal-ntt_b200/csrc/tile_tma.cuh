@@ -279,7 +279,13 @@ struct TPass {
   // staged twiddle bytes in shared memory, CTAs per SM
   static constexpr uint32_t SMEM_TW_BYTES =
       LSTAGE ? (KD == Kind::S ? 2u * 8u * 32u * ((1u << P) - 1u) : 4u * TWORDS) : 8u * TW_ENTRIES;
-  static constexpr int kCtasPerSm = ((LSTAGE && KD == Kind::S) || NT > 512) ? 1 : 2;
+  // Strided passes of fewer than 8 layers have tiles of 2^(P+5) words and NT =
+  // 2^(P+1) threads: as many CTAs as make up the 1024 threads that 64 registers
+  // each allow (16 at most).  With two CTAs of 128 threads per SM the 6-layer
+  // passes of the 2^18 x 100 natural-order LDE took 101 and 201 us (2.1 TB/s),
+  // with eight 54 and 102 us (4 TB/s).
+  static constexpr int kCtasPerSm =
+      ((LSTAGE && KD == Kind::S) || NT > 512) ? 1 : NT == 512 ? 2 : (1024 / NT < 16 ? 1024 / NT : 16);
   // Tile buffers of the whole-tile pipeline (run): three -- the tiles two and
   // one ahead in flight while one is computed -- for the staged strided passes
   // (one CTA per SM, 227 KiB with the twiddle chunks: 2^20 x 256 natural-order
