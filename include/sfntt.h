@@ -212,7 +212,9 @@ int sfntt_from_monty_dev(sfntt_ctx *ctx, int field, uint32_t *d_data, size_t len
  * (len = 2 * (batch << log_n) words).  The Circle NTT of a CM31 column is the
  * Circle NTT of its real parts plus i times that of its imaginary parts (the
  * twiddles lie in M31), with the M31 conventions (forward: bit-reversed out;
- * inverse: times n^-1).  The device calls use a context scratch of
+ * inverse: times n^-1).  The device calls need the twiddles and, for shapes
+ * that do not run on the interleaved words (buffers that are only 8-byte
+ * aligned, n < 32, small batches that fill no tile), a context scratch of
  * 8 * (batch << log_n) bytes: call sfntt_cm31_prepare before a graph capture. */
 int sfntt_cm31_prepare(sfntt_ctx *ctx, uint32_t log_n, uint32_t batch);
 int sfntt_cm31_ntt_dev(sfntt_ctx *ctx, int inverse, uint32_t *d_pairs, uint32_t log_n, uint32_t batch,

@@ -201,6 +201,10 @@ Status layers_dev(sfntt_ctx* ctx, int field, bool inverse, const uint32_t* in, u
                   uint64_t out_stride, uint32_t log_n, uint32_t batch, uint32_t a, uint32_t b, uint32_t scale_w,
                   const uint2* tw, cudaStream_t stream, const uint2* edge_twist = nullptr,
                   uint32_t edge_mask = 0);
+// The M31 network on dense columns of interleaved pairs, in place (ntt.cu);
+// *done = false: shape not supported, nothing launched.
+Status m31_pairs_dev(sfntt_ctx* ctx, bool inverse, uint32_t* d, uint32_t log_n, uint32_t batch, uint32_t scale_w,
+                     const uint2* tw, cudaStream_t stream, bool* done);
 // One-launch NTT of 2^13 .. 2^16-point columns on a thread-block cluster
 // (cluster_ntt.cu), in place on dense columns; fits: shape, alignment and at
 // most one wave of CTAs.

@@ -5,9 +5,13 @@
 // a #[repr(C)] struct of two M31 newtypes.  The Circle NTT's twiddles lie in
 // the base field, so the transform of a CM31 column is the base-field
 // transform of its real part plus i times that of its imaginary part.  The
-// batch of CM31 columns is split into 2 * batch base-field columns (real parts
-// first), run through the batched M31 engine, and merged back: split and merge
-// each read and write every word once with 8-byte / 4-byte coalesced accesses.
+// tile engine runs it on the interleaved words (m31_pairs_dev: word position =
+// 2 position + component, the layers one bit higher), in place and without the
+// two extra passes over memory of a split into planes: 2^16 x 24 30 -> 22 us
+// per transform, 2^20 x 8 143 -> 87 us, 2^12 x 1 9.3 -> 6.0 us.  Shapes outside
+// that engine (16-byte misaligned buffers, small ragged batches, n < 32) are
+// split into 2 * batch base-field columns (real parts first), run through the
+// batched M31 engine, and merged back.
 #include <algorithm>
 
 #include "context.hpp"
@@ -66,6 +70,11 @@ Status cm31_ntt_dev(sfntt_ctx* ctx, bool inverse, uint32_t* d_pairs, uint32_t lo
   if (((uint64_t)batch << log_n) >= (1ull << 39)) return {SFNTT_INVALID_SIZE, "too large"};
   if (!d_pairs) return {SFNTT_INVALID_ARGUMENT, "null buffer"};
   if (reinterpret_cast<uintptr_t>(d_pairs) & 7u) return {SFNTT_INVALID_ARGUMENT, "CM31 pairs must be 8-byte aligned"};
+  const uint2* tw = nullptr;
+  SFNTT_TRY(m31_twiddles(ctx, inverse, log_n, s, &tw));
+  bool done = false;
+  SFNTT_TRY(m31_pairs_dev(ctx, inverse, d_pairs, log_n, batch, inverse ? inv_n_of(SFNTT_M31, log_n) : 0u, tw, s, &done));
+  if (done) return {};
   uint32_t* planes = nullptr;
   SFNTT_TRY(cm31_scratch(ctx, log_n, batch, s, &planes));
   const uint64_t total = (uint64_t)batch << log_n;

@@ -151,6 +151,40 @@ Status layers_dev(sfntt_ctx* ctx, int field, bool inverse, const uint32_t* in, u
   return {};
 }
 
+// The M31 network on `batch` dense columns of 2^log_n interleaved pairs
+// (CM31), in place; *done stays false (nothing launched) where the shape does
+// not allow it.  A pair's two words sit at neighbouring positions and take the
+// same butterflies, so the passes run on the 2 n words of a column with the
+// layers one bit higher.
+Status m31_pairs_dev(sfntt_ctx* ctx, bool inverse, uint32_t* d, uint32_t log_n, uint32_t batch, uint32_t scale_w,
+                     const uint2* tw, cudaStream_t s, bool* done) {
+  *done = false;
+  uint32_t lo[4], cnt[4];
+  const int kt = ctx->no_tma ? 0 : tma_split(0, log_n, lo, cnt, ctx->split_c12, 12u);
+  TmaRequest req[4];
+  for (int i = 0; i < kt; ++i) {
+    const int pi = inverse ? i : (kt - 1 - i);
+    TmaRequest& r = req[i];
+    r.in = d;
+    r.out = d;
+    r.in_stride = r.out_stride = 2ull << log_n;
+    r.tw = tw;
+    r.log_n = log_n;
+    r.lo = lo[pi];
+    r.P = (int)cnt[pi];
+    r.contiguous = lo[pi] == 0;
+    r.batch = batch;
+    r.scale_w = (i == kt - 1) ? scale_w : 0u;
+    r.pair = true;
+    r.lstage = r.contiguous && log_n >= 12 && batch >= 16;
+    if (!tma_pass_ok(r)) return {};
+  }
+  if (kt == 0) return {};
+  for (int i = 0; i < kt; ++i) SFNTT_TRY(run_tma_pass_field(ctx, SFNTT_M31, !inverse, req[i], s));
+  *done = true;
+  return {};
+}
+
 // ---------------------------------------------------------------- V1 / V3 ---
 // One radix-2 layer over all columns: the per-layer dispatch of the
 // reference's V1 (src/ntt/*/metal_ct_dit_r2.rs) and, out of place, V3

@@ -39,7 +39,9 @@
 
 namespace sfntt {
 
-enum class Kind : int { C = 0, S = 1 };
+// Kind::D (tile_tma.cuh only): Kind::C on columns of interleaved pairs -- tile
+// bit 0 selects the pair's word, the group's bits start at tile bit 1.
+enum class Kind : int { C = 0, S = 1, D = 2 };
 
 // Rounds: P layers split into K = ceil(P / R) rounds, the first P % K rounds
 // one layer longer.  Round k covers group bits [b(k), b(k) + r(k)).
@@ -94,7 +96,7 @@ __host__ __device__ constexpr int filler_hint(int k, int i) {
 template <Kind KD, int P, int LT, int R>
 __host__ __device__ constexpr RoundMap make_map(int k) {
   constexpr int CB = P + LT;
-  constexpr int EOFF = (KD == Kind::S) ? LT : 0;
+  constexpr int EOFF = (KD == Kind::S) ? LT : (KD == Kind::D) ? 1 : 0;
   RoundMap m{};
   const int r = Plan<P, R>::r(k);
   const int b = Plan<P, R>::b(k);

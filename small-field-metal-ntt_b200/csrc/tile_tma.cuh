@@ -2,6 +2,8 @@
 //
 // Every tile is 2^13 words = 32 KiB = 256 rows of 128 bytes:
 //   Kind::C  2^13 consecutive words (2^(13-P) whole groups of 2^P points);
+//   Kind::D  (M31) the same on columns of interleaved pairs (CM31): word bit 0
+//            is the pair's component, the layers act on the bits above it;
 //   Kind::S  32 consecutive low positions (one 128-byte row each) of a
 //            2^P-point group with stride 2^lo, P <= 8 (one TMA box {32,1,2^P}).
 // Each CTA owns a strided sequence of tiles.  Thread 0 keeps one tile in
@@ -56,6 +58,8 @@ struct TmaArgs {
   uint32_t log_tpc;    // Kind::C: log2(tiles per column) (n >= 2^13)
   uint32_t batch;
   uint32_t spans;      // Kind::C: tiles span columns (n < 2^13, dense columns)
+  uint32_t pair;       // 1: columns of interleaved pairs (word position = 2 position + component;
+                       // log_n, lo and the twiddles count pairs)
   uint32_t scale, scale_w, scale_ws;
   int* err;
   // four-step twist applied at this pass's boundary (BabyBear): forward
@@ -117,22 +121,26 @@ struct TPass {
   // a position from the thread alone: with P = 8 every slot bit of both rounds
   // is a layer bit above the lanes).  M31 contiguous tiles (any layer
   // count): the per-block twiddles of the tile's 2^13 positions.
+  static constexpr bool CT = KD != Kind::S;                // contiguous tiles
+  static constexpr uint32_t PB = KD == Kind::D ? 1u : 0u;  // word bits below the positions
+  static_assert(KD != Kind::D || (!F::kMontgomery && !TW && !PLAIN && !HALVES && P <= 12), "pairs: M31 contiguous tiles");
   static_assert(!LSTAGE || (KD == Kind::S && F::kMontgomery && !PLAIN && P == 8) ||
-                    (KD == Kind::C && !F::kMontgomery && !TW),
+                    (CT && !F::kMontgomery && !TW),
                 "position staging: BabyBear 8-layer strided or M31 contiguous tiles");
   // Tile bits: 2^13-word tiles, except the 14-layer contiguous pass, whose
   // tile is one 2^14-point group (64 KiB, 1024 threads, one CTA per SM).
   static_assert(TBX == 0 || (KD == Kind::C && TBX >= P && !LSTAGE && !HALVES && !TW), "own tile size: whole columns");
   static constexpr int TB = TBX ? TBX : (KD == Kind::C && P > kTileBits) ? P : kTileBits;
-  static constexpr int LT = (KD == Kind::C) ? (TB - P) : 5;
+  static constexpr int LT = CT ? (TB - P) : 5;
   static constexpr int CB = P + LT;
   static constexpr int R = 4;
   static constexpr int NT = 1 << (CB - R);
   static constexpr int E = 1 << R;
   static constexpr int K = Plan<P, R>::K;
-  static_assert(KD == Kind::C ? (CB == TB && P <= 14) : (P <= 8), "tile shape");
+  static_assert(CT ? (CB == TB && P <= 14) : (P <= 8), "tile shape");
   static constexpr uint32_t TWORDS = 1u << CB;
   static constexpr uint32_t TBYTES = 4u << CB;
+  static constexpr uint32_t TPOS = TWORDS >> PB;  // positions of a contiguous tile
 
   using Geo = TileCoord;
 
@@ -140,21 +148,21 @@ struct TPass {
   // chunk, then high block.
   __device__ static __forceinline__ Geo geo(const TmaArgs& a, uint32_t t) {
     Geo g{};
-    if constexpr (KD == Kind::C) {
+    if constexpr (CT) {
       if (a.spans) {
         g.pos_base = 0;
         g.c1 = (int32_t)(t << (CB - 5));
         g.c2 = 0;
       } else {
         const uint32_t r = t & ((1u << a.log_tpc) - 1u);
-        g.pos_base = r << CB;
+        g.pos_base = r * TPOS;
         g.c1 = (int32_t)(r << (CB - 5));
         g.c2 = (int32_t)(t >> a.log_tpc);
       }
     } else {
       const uint32_t tt = t / a.batch;
       const uint32_t col = t - tt * a.batch;
-      const uint32_t lbits = a.lo - 5;
+      const uint32_t lbits = a.lo + a.pair - 5;
       const uint32_t lchunk = tt & ((1u << lbits) - 1u);
       g.hb = tt >> lbits;
       g.pos_base = lchunk << 5;
@@ -174,9 +182,9 @@ struct TPass {
       return geo(a, t);
     } else {
       Geo g{};
-      if constexpr (KD == Kind::C) {  // n >= 2^13 (never spanning)
+      if constexpr (CT) {  // n >= 2^13 (never spanning)
         const uint32_t r = t / a.batch;
-        g.pos_base = r << CB;
+        g.pos_base = r * TPOS;
         g.c1 = (int32_t)(r << (CB - 5));
         g.c2 = (int32_t)(t - r * a.batch);
       } else {
@@ -200,17 +208,17 @@ struct TPass {
 
   // 128-byte rows of spanning columns (one long column of batch << log_n words).
   __device__ static __forceinline__ int32_t span_rows(const TmaArgs& a) {
-    return (KD == Kind::C && a.spans) ? (int32_t)(((uint64_t)a.batch << a.log_n) >> 5) : INT32_MAX;
+    return (CT && a.spans) ? (int32_t)(((uint64_t)a.batch << (a.log_n + PB)) >> 5) : INT32_MAX;
   }
 
   __device__ static __forceinline__ void tma_load(const CUtensorMap* m, const Geo& g, uint32_t* dst, uint64_t* bar) {
-    if constexpr (KD == Kind::C) c_load(m, g.c1, g.c2, dst, bar, true);
+    if constexpr (CT) c_load(m, g.c1, g.c2, dst, bar, true);
     else tma::load_5d(dst, m, 0, g.s1, 0, g.s3, g.s4, bar);
   }
 
   __device__ static __forceinline__ void tma_store(const CUtensorMap* m, const Geo& g, const uint32_t* src,
                                                    int32_t rows = INT32_MAX) {
-    if constexpr (KD == Kind::C) c_store(m, g.c1, g.c2, src, true, rows);
+    if constexpr (CT) c_store(m, g.c1, g.c2, src, true, rows);
     else tma::store_5d(m, 0, g.s1, 0, g.s3, g.s4, src);
   }
 
@@ -278,7 +286,7 @@ struct TPass {
   static constexpr uint32_t CTILE_ENTRIES = 8190u;
   // staged twiddle bytes in shared memory, CTAs per SM
   static constexpr uint32_t SMEM_TW_BYTES =
-      LSTAGE ? (KD == Kind::S ? 2u * 8u * 32u * ((1u << P) - 1u) : 4u * TWORDS) : 8u * TW_ENTRIES;
+      LSTAGE ? (KD == Kind::S ? 2u * 8u * 32u * ((1u << P) - 1u) : 4u * TPOS) : 8u * TW_ENTRIES;
   // Strided passes of fewer than 8 layers have tiles of 2^(P+5) words and NT =
   // 2^(P+1) threads: as many CTAs as make up the 1024 threads that 64 registers
   // each allow (16 at most).  With two CTAs of 128 threads per SM the 6-layer
@@ -325,7 +333,7 @@ struct TPass {
 
   // Tile bits that are positions in a column (the rest select the column).
   __device__ static __forceinline__ uint32_t col_mask(const TmaArgs& a) {
-    return (TBX ? (1u << P) : (1u << a.log_n)) - 1u;
+    return (TBX ? (1u << P) : (1u << (a.log_n + PB))) - 1u;
   }
 
   // ---- twiddles: per-layer base pointer + compile-time offset per slot ----
@@ -346,10 +354,10 @@ struct TPass {
     } else if constexpr (LSTAGE && KD == Kind::S) {  // tw[L][pos mod 2^L] from the chunk's staged copy
       const uint32_t em = (1u << beta) - 1u;
       return tws[32u * em + ((((ct >> 5) & em) + ((cm >> 5) & em)) << 5) + (ct & 31u)];
-    } else if constexpr (LSTAGE && KD == Kind::C) {  // M31: the tile's staged table-order copy (w' = 2w + (w >> 30))
+    } else if constexpr (LSTAGE && CT) {  // M31: the tile's staged table-order copy (w' = 2w + (w >> 30))
       static_assert(!kStageThreadOrder, "12-layer rounds take their staged twiddles in round()");
-      const uint32_t* tw32 = reinterpret_cast<const uint32_t*>(tws) + (TWORDS - (TWORDS >> L));
-      const uint32_t ws = tw32[(ct >> (L + 1)) + (cm >> (L + 1))];
+      const uint32_t* tw32 = reinterpret_cast<const uint32_t*>(tws) + (TPOS - (TPOS >> L));
+      const uint32_t ws = tw32[(ct >> (L + 1 + PB)) + (cm >> (L + 1 + PB))];
       return make_uint2(ws >> 1, ws);
     } else if constexpr (F::kMontgomery) {  // BabyBear strided, per position: tw[L][pos mod 2^L]
       const uint2* base = a.tw + ((1u << L) - 1u);
@@ -359,8 +367,9 @@ struct TPass {
     } else {  // M31: tw[L][pos >> (L+1)]
       const uint32_t n = 1u << a.log_n;
       const uint2* base = a.tw + (n - (n >> L));
-      if constexpr (KD == Kind::C) {  // tile bits above log n select the column (spanning tiles)
-        return __ldg(base + ((g.pos_base >> (L + 1)) + ((ct & col_mask(a)) >> (L + 1)) + ((cm & col_mask(a)) >> (L + 1))));
+      if constexpr (CT) {  // tile bits above log n select the column (spanning tiles)
+        return __ldg(base + ((g.pos_base >> (L + 1)) + ((ct & col_mask(a)) >> (L + 1 + PB)) +
+                             ((cm & col_mask(a)) >> (L + 1 + PB))));
       } else {
         return __ldg(base + ((g.hb << (P - beta - 1)) + ((ct >> 5) >> (beta + 1)) + ((cm >> 5) >> (beta + 1))));
       }
@@ -389,7 +398,7 @@ struct TPass {
         uint2 tv[E / 2];
         if constexpr (LSTAGE) {
           // this thread's 2^(r-1-j) twiddles of layer j (a constant once unrolled)
-          const uint32_t* tw32 = reinterpret_cast<const uint32_t*>(tws) + (TWORDS - (TWORDS >> L));
+          const uint32_t* tw32 = reinterpret_cast<const uint32_t*>(tws) + (TPOS - (TPOS >> L));
           if constexpr (k == 0 && kStageThreadOrder) {  // thread-ordered first-round layers
             switch (r - 1 - j) {
               case 3: staged_w<4, 0>(tw32 + 4u * tid, tv); staged_w<4, 4>(tw32 + 4u * (NT + tid), tv); break;
@@ -398,7 +407,7 @@ struct TPass {
               default: staged_w<1, 0>(tw32 + tid, tv); break;
             }
           } else {
-            const uint32_t* p = tw32 + (ct >> (L + 1));
+            const uint32_t* p = tw32 + (ct >> (L + 1 + PB));
             switch (r - 1 - j) {
               case 3: staged_w<4, 0>(p, tv); staged_w<4, 4>(p + 4, tv); break;
               case 2: staged_w<4, 0>(p, tv); break;
@@ -428,7 +437,7 @@ struct TPass {
           }
           if (!copied) {
             const uint2* base = a.tw + (n - (n >> L));
-            if constexpr (KD == Kind::C) base += (g.pos_base >> (L + 1)) + ((ct & col_mask(a)) >> (L + 1));
+            if constexpr (CT) base += (g.pos_base >> (L + 1)) + ((ct & col_mask(a)) >> (L + 1 + PB));
             else base += (g.hb << (P - beta - 1)) + ((ct >> 5) >> (beta + 1));
             if (j == r - 1) {
               tv[0] = __ldg(base);
@@ -524,7 +533,7 @@ struct TPass {
 
   // Shared-memory word of tile word c (the TMA layout of this tile kind: the
   // row order of c_row_perm, then the swizzle).
-  static constexpr bool kSwz = (KD == Kind::C) && kSwizzleC;
+  static constexpr bool kSwz = CT && kSwizzleC;
   static constexpr bool kRowPerm = (KD == Kind::C) && c_row_perm(P);
   __host__ __device__ static constexpr uint32_t lay(uint32_t c) {
     // rows [c5 c6][c8 .. c(TB-2)][c7][c(TB-1)]
@@ -732,7 +741,7 @@ struct TPass {
   __device__ static __forceinline__ uint32_t pos_of(const TmaArgs& a, const Geo& g, uint32_t ct, int m) {
     using M = RM<KD, P, LT, R, k>;
     const uint32_t cm = M::cm(m);
-    if constexpr (KD == Kind::C) return g.pos_base + ct + cm;
+    if constexpr (CT) return g.pos_base + ct + cm;
     else
       return (g.hb << (a.lo + P)) + g.pos_base + (ct & 31u) + (cm & 31u) + (((ct >> 5) + (cm >> 5)) << a.lo);
   }
@@ -839,17 +848,17 @@ struct TPass {
   static_assert(!HALVES || halves_ok(), "independent halves: contiguous tiles whose top bit is thread bit 8");
   static constexpr uint32_t HWORDS = TWORDS / 2, HBYTES = TBYTES / 2, HROWS = HWORDS / 32;
 
-  // M31 per-block twiddles (Shoup companions) of every layer L < P over tile
-  // positions [pos_base, pos_base + 2^CB), all in table order: 2^(CB-1-L)
-  // consecutive entries of layer L at 2^CB - (2^CB >> L).
+  // M31 per-block twiddles (Shoup companions) of every layer L < P over the
+  // tile's TPOS positions from pos_base on, all in table order: TPOS / 2^(L+1)
+  // consecutive entries of layer L at TPOS - (TPOS >> L).
   __device__ static __forceinline__ void stage_ctile_plain(uint32_t* dst, const TmaArgs& a, uint32_t pos_base,
                                                            uint32_t tid) {
     const uint32_t n = 1u << a.log_n;
-    const uint32_t end = TWORDS - (TWORDS >> P);
+    const uint32_t end = TPOS - (TPOS >> P);
     for (uint32_t e = tid; e < end; e += NT) {
-      // e in [2^CB - 2^(CB-L), 2^CB - 2^(CB-1-L))
-      const uint32_t L = (uint32_t)(CB - 1) - (31u - __clz(TWORDS - 1u - e));
-      const uint32_t local = e - (TWORDS - (TWORDS >> L));
+      // e in [TPOS - (TPOS >> L), TPOS - (TPOS >> (L+1)))
+      const uint32_t L = (uint32_t)(CB - 1) - PB - (31u - __clz(TPOS - 1u - e));
+      const uint32_t local = e - (TPOS - (TPOS >> L));
       dst[e] = __ldg(&a.tw[(n - (n >> L)) + (pos_base >> (L + 1)) + local].y);
     }
   }
@@ -989,11 +998,11 @@ struct TPass {
         // Every thread passed the previous tile's pre-store barrier after its
         // last twiddle read; the barrier here publishes the new copy (the
         // positions are a function of t, the same for the whole CTA).
-        const uint32_t key = (KD == Kind::C) ? g.pos_base : ((uint32_t)g.s1 >> 1);
+        const uint32_t key = CT ? g.pos_base : ((uint32_t)g.s1 >> 1);
         if (key != staged) {
           if constexpr (kStageThreadOrder) {
             stage_ctile(reinterpret_cast<uint32_t*>(tws), a, g.pos_base, tid);
-          } else if constexpr (KD == Kind::C) {
+          } else if constexpr (CT) {
             stage_ctile_plain(reinterpret_cast<uint32_t*>(tws), a, g.pos_base, tid);
           } else {  // both chunks of the pair
             stage_lchunk(tws, a.tw, a.lo, 2u * key, tid);

@@ -28,6 +28,9 @@ struct TmaRequest {
   // per-position twiddles staged in shared memory, one CTA per SM walking the
   // columns (BabyBear 8-layer strided or M31 contiguous passes, n >= 2^13)
   bool lstage = false;
+  // M31 over columns of interleaved pairs (CM31): log_n, lo and P count pairs,
+  // the strides words
+  bool pair = false;
 };
 
 // Resolved once through the runtime (no link-time dependency on libcuda).
@@ -48,15 +51,16 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // 7.6 against 5.9 us).
 inline bool tma_pass_ok(const TmaRequest& r) {
   if (!aligned16(r.in) || !aligned16(r.out) || (r.in_stride & 3) || (r.out_stride & 3)) return false;
-  const uint64_t n = 1ull << r.log_n;
+  const uint32_t pair = r.pair ? 1u : 0u;
+  const uint64_t n = 1ull << (r.log_n + pair);  // words per column
   if (r.contiguous) {
-    if (r.P < 5 || r.P > 14 || r.lo != 0) return false;
+    if (r.P < 5 || r.P > (r.pair ? 12 : 14) || r.lo != 0) return false;
     if (n >= kTileWords) return true;
     const uint64_t words = (uint64_t)r.batch * n;
     return n >= 32 && r.in_stride == n && r.out_stride == n &&
-           (words % kTileWords == 0 || words >= (r.log_n >= 12 ? (uint64_t)kTileWords : 1ull << 18));
+           (words % kTileWords == 0 || words >= (r.log_n + pair >= 12 ? (uint64_t)kTileWords : 1ull << 18));
   }
-  return r.P >= 1 && r.P <= 8 && r.lo >= 5 && r.lo + r.P <= r.log_n;
+  return r.P >= 1 && r.P <= 8 && r.lo + pair >= 5 && r.lo + r.P <= r.log_n;
 }
 
 // Contiguous tiles of a P-layer pass.  Row order (c_row_perm(P) false):
@@ -98,7 +102,7 @@ inline Status encode_s_map(CUtensorMap* m, const uint32_t* base, uint32_t lo, in
 template <class F, bool DESC, Kind KD, int P, bool PLAIN, bool TW, bool LSTAGE>
 const char* tma_pass_name() {
   static const std::string nm = std::string(F::kTag) + "_" + (DESC ? "fwd" : "inv") +
-                                "_tma_" + (KD == Kind::C ? "C" : "S") + std::to_string(P) + (PLAIN ? "p" : "") +
+                                "_tma_" + (KD == Kind::C ? "C" : KD == Kind::D ? "D" : "S") + std::to_string(P) + (PLAIN ? "p" : "") +
                                 (TW ? "t" : "") + (LSTAGE ? "c" : "");
   return nm.c_str();
 }
@@ -106,9 +110,12 @@ const char* tma_pass_name() {
 template <class F, bool DESC, Kind KD, int P, bool PLAIN, bool TW, bool LSTAGE = false, bool HALVES = false>
 Status launch_tma_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
   using T = TPass<F, DESC, KD, P, PLAIN, TW, LSTAGE, HALVES>;
-  const uint64_t n = 1ull << r.log_n;
+  const uint32_t pair = r.pair ? 1u : 0u;
+  const uint32_t log_w = r.log_n + pair, lo_w = r.lo + pair;  // in words
+  const uint64_t n = 1ull << log_w;
   CUtensorMap min, mout;
   TmaArgs a{};
+  a.pair = pair;
   a.tw = r.tw;
   a.log_n = r.log_n;
   a.lo = r.lo;
@@ -120,19 +127,20 @@ Status launch_tma_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
   a.twist = r.twist;
   a.twist_mask = r.twist_mask;
   a.twist_compact = r.twist_compact ? 1u : 0u;
-  if constexpr (KD == Kind::C) {
+  if constexpr (KD != Kind::S) {
     const uint32_t rows = HALVES ? T::HROWS : T::TWORDS / 32;
-    SFNTT_TRY(encode_c_map(&min, r.in, r.log_n, r.in_stride, r.batch, P, rows));
-    SFNTT_TRY(encode_c_map(&mout, r.out, r.log_n, r.out_stride, r.batch, P, rows));
+    const int order = KD == Kind::C ? P : 0;  // rows of pair tiles stay in order
+    SFNTT_TRY(encode_c_map(&min, r.in, log_w, r.in_stride, r.batch, order, rows));
+    SFNTT_TRY(encode_c_map(&mout, r.out, log_w, r.out_stride, r.batch, order, rows));
     a.spans = n < T::TWORDS;
-    a.log_tpc = a.spans ? 0u : r.log_n - T::CB;
+    a.log_tpc = a.spans ? 0u : log_w - T::CB;
     // every M31 table with n >= 2^13 carries its first-round copy from entry n on
     if constexpr (T::kRound0Copy) a.tw0 = a.spans ? nullptr : r.tw + n;
     a.ntiles = (uint32_t)(((uint64_t)r.batch * n + T::TWORDS - 1) >> T::CB);
   } else {
-    const uint64_t hb = n >> (r.lo + P);
-    SFNTT_TRY(encode_s_map(&min, r.in, r.lo, P, hb, 1ull << (r.lo + P), r.in_stride, r.batch));
-    SFNTT_TRY(encode_s_map(&mout, r.out, r.lo, P, hb, 1ull << (r.lo + P), r.out_stride, r.batch));
+    const uint64_t hb = n >> (lo_w + P);
+    SFNTT_TRY(encode_s_map(&min, r.in, lo_w, P, hb, 1ull << (lo_w + P), r.in_stride, r.batch));
+    SFNTT_TRY(encode_s_map(&mout, r.out, lo_w, P, hb, 1ull << (lo_w + P), r.out_stride, r.batch));
     a.ntiles = (uint32_t)(((uint64_t)r.batch * n) >> (P + 5));
   }
   constexpr int smem = T::kSmemBytes;
@@ -144,7 +152,7 @@ Status launch_tma_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
   launch_begin(ctx, s);
   SFNTT_CU(launch_pdl(kern, grid, T::NT, smem, s, pdl_fits(grid), min, mout, a));
   return launch_check(ctx, tma_pass_name<F, DESC, KD, P, PLAIN, TW, LSTAGE>(), s,
-                      ((uint64_t)r.batch << r.log_n) * 8u);
+                      ((uint64_t)r.batch << log_w) * 8u);
 }
 
 // BabyBear and KoalaBear instantiate the twist / plain variants; M31 never needs them.
@@ -175,9 +183,25 @@ Status launch_tma_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
     }                                                                                            \
     return launch_tma_pass<F, DESC, Kind::S, PP, false, false>(ctx, r, s);
 
+#define SFNTT_TMA_D(PP)                                                                          \
+  case PP:                                                                                       \
+    if (r.lstage && r.log_n + 1 >= kTileBits)                                                    \
+      return launch_tma_pass<F, DESC, Kind::D, PP, false, false, true>(ctx, r, s);               \
+    return launch_tma_pass<F, DESC, Kind::D, PP, false, false>(ctx, r, s);
+
 template <class F, bool DESC>
 Status run_tma_pass_impl(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
   if (!tma_pass_ok(r)) return {SFNTT_INVALID_ARGUMENT, "pass shape not supported by the TMA engine"};
+  if (r.pair && F::kMontgomery) return {SFNTT_INVALID_ARGUMENT, "passes over pairs are M31"};
+  if constexpr (!F::kMontgomery) {
+    if (r.pair && r.contiguous) {
+      switch (r.P) {
+        SFNTT_TMA_D(5) SFNTT_TMA_D(6) SFNTT_TMA_D(7) SFNTT_TMA_D(8)
+        SFNTT_TMA_D(9) SFNTT_TMA_D(10) SFNTT_TMA_D(11) SFNTT_TMA_D(12)
+        default: break;
+      }
+    }
+  }
   if (!F::kMontgomery && (r.twist || r.plain)) return {SFNTT_INVALID_ARGUMENT, "M31 passes take no twist"};
   if (r.contiguous) {
     switch (r.P) {
@@ -197,6 +221,7 @@ Status run_tma_pass_impl(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
 }
 #undef SFNTT_TMA_C
 #undef SFNTT_TMA_S
+#undef SFNTT_TMA_D
 
 Status run_tma_pass_bb_fwd(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s);
 Status run_tma_pass_bb_inv(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s);
