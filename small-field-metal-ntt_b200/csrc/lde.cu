@@ -209,6 +209,42 @@ Status launch_tma_expand(sfntt_ctx* ctx, const uint32_t* src, uint64_t src_strid
   return launch_check(ctx, name.c_str(), s, ((uint64_t)batch * n) * 4u * (1u + (1u << added_bits)));
 }
 
+// The M31 expansion on warp-owned tiles, up to 4x (each output block's
+// twiddles sit in shared memory) and from three tiles per SM on (tile_warp.cuh).
+__global__ void __launch_bounds__(wt::kThreads, wt::kCtasPerSm)
+warp_expand_m31_kernel(const __grid_constant__ CUtensorMap min, const __grid_constant__ CUtensorMap mout, TmaArgs a) {
+  pdl_enter();
+  WExpandM31::run(&min, &mout, a);
+}
+
+Status launch_warp_expand_m31(sfntt_ctx* ctx, uint32_t* d_out, uint32_t log_n, uint32_t batch, uint32_t added_bits,
+                              const uint2* tw_inv, const uint2* tw_fwd, uint32_t scale_w, cudaStream_t s) {
+  using X = WExpandM31;
+  const uint32_t lo = log_n - 8;
+  const uint64_t n = 1ull << log_n, n_ext = n << added_bits;
+  CUtensorMap min, mout;
+  SFNTT_TRY(encode_w_map(&min, d_out, lo, wt::kSwapped, 1, n, n_ext, batch));
+  SFNTT_TRY(encode_w_map(&mout, d_out, lo, wt::kSwapped, 1ull << added_bits, n, n_ext, batch));
+  TmaArgs a{};
+  a.tw = tw_inv;
+  a.tw_fwd = tw_fwd;
+  a.log_n = log_n;
+  a.lo = lo;
+  a.batch = batch;
+  a.log_q = added_bits;
+  a.err = ctx->err.as<int>();
+  a.ntiles = (uint32_t)(((uint64_t)batch * n) >> kTileBits);
+  a.scale_w = scale_w;
+  a.scale_ws = (uint32_t)(((uint64_t)scale_w << 32) / M31::P);
+  static std::atomic<uint64_t> smem_done{0};
+  SFNTT_TRY(smem_limit_once(warp_expand_m31_kernel, X::kSmemBytes, ctx->device, smem_done));
+  const uint32_t ctas = ctx->tma_ctas > 0 ? std::min<uint32_t>((uint32_t)ctx->tma_ctas, wt::kCtasPerSm) : wt::kCtasPerSm;
+  const uint32_t grid = std::min<uint32_t>(a.ntiles, ctas * (uint32_t)ctx->sm_count);
+  launch_begin(ctx, s);
+  SFNTT_CU(launch_pdl(warp_expand_m31_kernel, grid, wt::kThreads, X::kSmemBytes, s, pdl_fits(grid), min, mout, a));
+  return launch_check(ctx, "m31_lde_expand_warp_S8", s, ((uint64_t)batch * n) * 4u * (1u + (1u << added_bits)));
+}
+
 // The natural-order expansion (TExpandC): src holds the inverse layers
 // [12, log_n) of every column (stride n); d_out receives the 2x extension with
 // the DIT layers [0, 12) of both interleaved cosets done.
@@ -451,8 +487,11 @@ Status m31_lde_dev(sfntt_ctx* ctx, const uint32_t* d_in, uint32_t* d_out, uint32
     // the extended network; F3: forward layers [0, lo) of the extended network.
     const uint32_t lo = log_n - 8;
     SFNTT_TRY(layers_dev(ctx, SFNTT_M31, true, d_in, d_out, n, n_ext, log_n, batch, 0, lo, 0u, tw_inv, s));
-    SFNTT_TRY((launch_tma_expand<M31, 8, false>(ctx, d_out, n_ext, d_out, log_n, batch, added_bits, tw_inv, tw_fwd,
-                                                nullptr, s, inv_n_of(SFNTT_M31, log_n))));
+    if (added_bits <= 2 && (((uint64_t)batch << log_n) >> kTileBits) >= 3ull * (uint64_t)ctx->sm_count)
+      SFNTT_TRY(launch_warp_expand_m31(ctx, d_out, log_n, batch, added_bits, tw_inv, tw_fwd, inv_n_of(SFNTT_M31, log_n), s));
+    else
+      SFNTT_TRY((launch_tma_expand<M31, 8, false>(ctx, d_out, n_ext, d_out, log_n, batch, added_bits, tw_inv, tw_fwd,
+                                                  nullptr, s, inv_n_of(SFNTT_M31, log_n))));
     return layers_dev(ctx, SFNTT_M31, false, d_out, d_out, n_ext, n_ext, log_ext, batch, 0, lo, 0u, tw_fwd, s);
   }
   if (log_n > 0) {

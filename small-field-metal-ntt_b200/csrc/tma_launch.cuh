@@ -8,6 +8,7 @@
 
 #include "context.hpp"
 #include "tile_tma.cuh"
+#include "tile_warp.cuh"
 
 namespace sfntt {
 
@@ -99,6 +100,55 @@ inline Status encode_s_map(CUtensorMap* m, const uint32_t* base, uint32_t lo, in
   return tensor_map_encode(m, base, 5, dims, strides, box);
 }
 
+// The same strided tiles of 8 layers for the warp-owned passes: positions as one
+// dimension, the element in two, in the row order of tile_warp.cuh.
+inline Status encode_w_map(CUtensorMap* m, const uint32_t* base, uint32_t lo, wt::RowOrder order, uint64_t hb_count,
+                           uint64_t hb_stride, uint64_t stride, uint32_t batch) {
+  const cuuint64_t elo = (4ull << lo), ehi = (64ull << lo);  // byte strides of e + 1, e + 16
+  const cuuint64_t dims[5] = {1ull << lo, 16, 16, hb_count, batch};
+  const cuuint64_t strides[4] = {order == wt::kSwapped ? ehi : elo, order == wt::kSwapped ? elo : ehi, hb_stride * 4,
+                                 stride * 4};
+  const cuuint32_t box[5] = {32, 16, 16, 1, 1};
+  return tensor_map_encode(m, base, 5, dims, strides, box, true);
+}
+
+// The passes that take the warp-owned tiles: the network's top 8 layers without
+// a boundary twist, at least three tiles per SM (see tile_warp.cuh).
+template <class F>
+bool warp_pass_ok(const sfntt_ctx* ctx, const TmaRequest& r) {
+  return (F::kMontgomery ? r.plain && !r.twist : !r.twist) && r.lo + 8 == r.log_n &&
+         (((uint64_t)r.batch << (r.log_n + (r.pair ? 1 : 0))) >> kTileBits) >= 3ull * (uint64_t)ctx->sm_count;
+}
+
+template <class F, bool DESC>
+Status launch_warp_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
+  using W = WPass<F, DESC>;
+  const uint32_t pair = r.pair ? 1u : 0u, log_w = r.log_n + pair, lo_w = r.lo + pair;
+  CUtensorMap min, mout;
+  SFNTT_TRY(encode_w_map(&min, r.in, lo_w, W::kIn, 1, 1ull << log_w, r.in_stride, r.batch));
+  SFNTT_TRY(encode_w_map(&mout, r.out, lo_w, W::kOut, 1, 1ull << log_w, r.out_stride, r.batch));
+  TmaArgs a{};
+  a.tw = r.tw;
+  a.log_n = r.log_n;
+  a.lo = r.lo;
+  a.pair = pair;
+  a.batch = r.batch;
+  a.err = ctx->err.as<int>();
+  a.scale = r.scale_w ? 1u : 0u;
+  a.scale_w = r.scale_w;
+  a.scale_ws = (uint32_t)(((uint64_t)r.scale_w << 32) / F::P);
+  a.ntiles = (uint32_t)(((uint64_t)r.batch << log_w) >> kTileBits);
+  auto kern = warp_pass_kernel<F, DESC>;
+  static std::atomic<uint64_t> smem_done{0};
+  SFNTT_TRY(smem_limit_once(kern, W::kSmemBytes, ctx->device, smem_done));
+  const uint32_t ctas = ctx->tma_ctas > 0 ? std::min<uint32_t>((uint32_t)ctx->tma_ctas, wt::kCtasPerSm) : wt::kCtasPerSm;
+  const uint32_t grid = std::min<uint32_t>(a.ntiles, ctas * (uint32_t)ctx->sm_count);
+  launch_begin(ctx, s);
+  SFNTT_CU(launch_pdl(kern, grid, wt::kThreads, W::kSmemBytes, s, pdl_fits(grid), min, mout, a));
+  static const std::string name = std::string(F::kTag) + (DESC ? "_fwd" : "_inv") + "_warp_S8" + (F::kMontgomery ? "p" : "");
+  return launch_check(ctx, name.c_str(), s, ((uint64_t)r.batch << log_w) * 8u);
+}
+
 template <class F, bool DESC, Kind KD, int P, bool PLAIN, bool TW, bool LSTAGE>
 const char* tma_pass_name() {
   static const std::string nm = std::string(F::kTag) + "_" + (DESC ? "fwd" : "inv") +
@@ -173,6 +223,9 @@ Status launch_tma_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
     return launch_tma_pass<F, DESC, Kind::C, PP, false, false>(ctx, r, s);
 #define SFNTT_TMA_S(PP)                                                                          \
   case PP:                                                                                       \
+    if constexpr (PP == 8) {                                                                     \
+      if (warp_pass_ok<F>(ctx, r)) return launch_warp_pass<F, DESC>(ctx, r, s);                  \
+    }                                                                                            \
     if constexpr (F::kMontgomery) {                                                              \
       if (r.plain && r.twist) return launch_tma_pass<F, DESC, Kind::S, PP, true, true>(ctx, r, s); \
       if (r.plain) return launch_tma_pass<F, DESC, Kind::S, PP, true, false>(ctx, r, s);         \
