@@ -1,16 +1,15 @@
 // cluster_ntt.cu -- one-launch NTT of columns of 2^13 .. 2^16 points on a
 // thread-block cluster.
 //
-// A column of n = 2^(12+X) points is split over CS = 2^(X-1) CTAs of one
-// cluster, CTA r owning the contiguous positions [r 2^13, (r+1) 2^13) in
-// shared memory.  Layers [0, 12) pair positions inside a 2^13-word block and
-// run on the tile engine's rounds (TPass<F, DESC, Kind::C, 12>: registers,
-// shared-memory exchanges, staged BabyBear twiddles or the M31 first-round
-// copy).  The X cross layers [12, 12+X) pair positions 2^12 apart: the points
-// {base + k 2^12 : k < 2^X} (base < 2^12) form one group, and each thread owns
+// A column of n = 2^(12+X) points is split over 2^X CTAs of one cluster (16 at
+// 2^16 points: the non-portable size), CTA r owning the contiguous positions
+// [r 2^12, (r+1) 2^12) in shared memory.  Layers [0, 12) pair positions inside a
+// block and run on the tile engine's rounds (TPass<F, DESC, Kind::C, 12> on
+// 2^12-word tiles, 256 threads: registers, shared-memory exchanges).  The X cross
+// layers [12, 12+X) pair positions 2^12 apart: the points {base + k 2^12 : k <
+// 2^X} (base < 2^12) form one group, one point per block, and each thread owns
 // 16 / 2^X whole groups, so these layers run in registers.  The exchange
-// between the two parts goes through distributed shared memory: point k of a
-// group lives in CTA k >> 1 at word base + (k & 1) 2^12.
+// between the two parts goes through distributed shared memory.
 //
 //   inverse (layers ascending): load the block, in-block layers, cluster
 //     barrier, gather the groups from the cluster's blocks, cross layers and
@@ -21,9 +20,17 @@
 //     into the owning blocks, cluster barrier, in-block layers, store the block.
 //
 // Every global read of a column happens before the cluster's first barrier and
-// every global write after it, so the transform works in place.  The
-// persistent TMA passes need two launches for these sizes (about 4.5 us each
-// for one column); this is one.
+// every global write after it, so the transform works in place.
+//
+// One column is a chain of latencies: 16 layers on the SMs of one cluster, the
+// twiddles' L2 latency and the launch.  Blocks of 2^12 words halve the work per
+// SM of 2^13-word ones, and the twiddles -- BabyBear / KoalaBear's in-block table
+// into shared memory, M31's 32 KiB of per-block twiddles into L1, the cross
+// twiddles into registers -- are fetched before the wait for the previous kernel
+// (programmatic dependent launch), so they overlap its end.  Forward / inverse of
+// one column from a graph, 2^13-word blocks with the twiddles fetched layer by
+// layer -> now: BabyBear 2^13 6.7 / 7.1 -> 4.0 / 4.5 us, 2^16 7.9 / 8.4 -> 5.0 /
+// 5.3 us; M31 2^13 6.1 / 6.0 -> 4.1 / 4.4 us, 2^16 7.2 / 7.4 -> 5.4 / 5.3 us.
 #include <cooperative_groups.h>
 
 #include "context.hpp"
@@ -37,42 +44,72 @@ namespace cg = cooperative_groups;
 
 template <class F, bool DESC, int X>
 struct ClusterNtt {
-  using TP = TPass<F, DESC, Kind::C, 12>;
-  static constexpr int CS = 1 << (X - 1);  // CTAs per column
-  static constexpr int G = 1 << X;         // points per cross group
+  using TP = TPass<F, DESC, Kind::C, 12, false, false, false, false, 12>;
+  static constexpr int CS = 1 << X;        // CTAs per column
+  static constexpr int G = 1 << X;         // points per cross group, one per block
   static constexpr int GPT = 16 / G;       // groups per thread
   static constexpr uint32_t NT = TP::NT;
   static constexpr uint32_t LOG_N = 12 + X;
   static constexpr uint32_t BASES = 4096u / CS;  // group bases per CTA
-  static_assert(NT == 512 && TP::E == 16 && BASES == GPT * NT, "one thread: 16 points in whole groups");
+  static_assert(NT == 256 && TP::E == 16 && BASES == GPT * NT && TP::TWORDS == 4096u,
+                "one thread: 16 points in whole groups");
+
+  // Butterflies of one group and layer j, low points in order: cross_at(k, j)
+  // numbers the twiddles a thread needs for one group (M31: 2^(X-1-j) per layer,
+  // the same for every group; BabyBear / KoalaBear: 2^j).
+  static constexpr int CT = G - 1;  // per group
+  static constexpr int CN = F::kMontgomery ? GPT * CT : CT;
+  __device__ static constexpr int cross_at(int k, int j) {
+    return F::kMontgomery ? ((1 << j) - 1) + (k & ((1 << j) - 1)) : (G - (G >> j)) + (k >> (j + 1));
+  }
 
   // Twiddle of the cross butterfly whose lower point is k (bit j clear) of the
   // group at `base`, layer L = 12 + j: BabyBear / KoalaBear tw[L][pos mod 2^L],
   // M31 tw[L][pos >> (L+1)] (the same for every base).
+  // A volatile load stays ahead of the wait for the previous kernel.
+  __device__ static __forceinline__ uint2 ld_tw(const uint2* p) {
+    uint2 r;
+    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+    return r;
+  }
   __device__ static __forceinline__ uint2 cross_tw(const uint2* tw, uint32_t base, int k, int j) {
     const uint32_t L = 12u + (uint32_t)j;
     if constexpr (F::kMontgomery) {
-      return __ldg(tw + ((1u << L) - 1u) + base + ((uint32_t)(k & ((1 << j) - 1)) << 12));
+      return ld_tw(tw + ((1u << L) - 1u) + base + ((uint32_t)(k & ((1 << j) - 1)) << 12));
     } else {
       const uint32_t n = 1u << LOG_N;
-      return __ldg(tw + (n - (n >> L)) + ((uint32_t)k >> (j + 1)));
+      return ld_tw(tw + (n - (n >> L)) + ((uint32_t)k >> (j + 1)));
     }
+  }
+
+  // Every cross twiddle of the thread's groups, all loads in flight at once.
+  __device__ static __forceinline__ void load_cross(uint2 (&t)[CN], uint32_t base0, const uint2* tw) {
+#pragma unroll
+    for (int gi = 0; gi < (F::kMontgomery ? GPT : 1); ++gi)
+#pragma unroll
+      for (int j = 0; j < X; ++j)
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+          if (k & (1 << j)) continue;
+          const int first = F::kMontgomery ? (k & ((1 << j) - 1)) : ((k >> (j + 1)) << (j + 1));
+          if (k == first) t[gi * CT + cross_at(k, j)] = cross_tw(tw, base0 + (uint32_t)gi * NT, k, j);
+        }
   }
 
   // The X cross layers on the thread's groups (forward: descending, inverse:
   // ascending, then n^-1); canonical values out.
-  __device__ static __forceinline__ void cross(uint32_t (&v)[16], uint32_t base0, const uint2* tw, uint32_t scale_w,
+  __device__ static __forceinline__ void cross(uint32_t (&v)[16], const uint2 (&t)[CN], uint32_t scale_w,
                                                uint32_t scale_ws) {
 #pragma unroll
     for (int gi = 0; gi < GPT; ++gi) {
-      const uint32_t base = base0 + (uint32_t)gi * NT;
 #pragma unroll
       for (int jj = 0; jj < X; ++jj) {
         const int j = DESC ? (X - 1 - jj) : jj;
 #pragma unroll
         for (int k = 0; k < G; ++k) {
           if (k & (1 << j)) continue;
-          butterfly<F, DESC>(v[gi * G + k], v[gi * G + (k | (1 << j))], cross_tw(tw, base, k, j));
+          butterfly<F, DESC>(v[gi * G + k], v[gi * G + (k | (1 << j))],
+                             t[(F::kMontgomery ? gi * CT : 0) + cross_at(k, j)]);
         }
       }
     }
@@ -86,7 +123,7 @@ struct ClusterNtt {
   __device__ static void run(uint32_t* d, const uint2* tw, uint32_t scale_w, uint32_t scale_ws) {
     extern __shared__ __align__(1024) uint32_t smem_words[];
     uint32_t* tile = smem_words;                                // the block, in TP's swizzled layout
-    uint2* tws = reinterpret_cast<uint2*>(tile + kTileWords);  // BabyBear / KoalaBear layers [0, 12)
+    uint2* tws = reinterpret_cast<uint2*>(tile + TP::TWORDS);  // the block's twiddles, layers [0, 12)
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank();
     const uint32_t tid = threadIdx.x;
@@ -98,11 +135,29 @@ struct ClusterNtt {
     a.lo = 0;
     a.batch = 1;
     a.log_tpc = (uint32_t)(X - 1);
-    if constexpr (TP::kRound0Copy) a.tw0 = tw + n;  // M31 tables with n >= 2^13 carry it
     TileCoord g{};
-    g.pos_base = rank << kTileBits;
-    if constexpr (TP::kStaged) TP::stage_twiddles(tws, tw, tid);
+    g.pos_base = rank << 12;
     const uint32_t base0 = rank * BASES + tid;  // group gi: base0 + gi NT
+    uint2 ctw[CN];
+    // The tables do not depend on the previous kernel: under programmatic
+    // dependent launch their loads overlap its end.
+    pdl_trigger();
+    if constexpr (TP::kStaged) {
+      TP::stage_twiddles(tws, tw, tid);
+    } else {
+      // layers 0..7 of the block are 255 lines of 128 bytes, one per thread;
+      // the last thread takes layer 8's 64 bytes and what follows them
+      const uint32_t L = tid < 255u ? 7u - (31u - __clz(255u - tid)) : 8u;
+      const char* p = reinterpret_cast<const char*>(tw + (n - (n >> L)) + (g.pos_base >> (L + 1)) +
+                                                    16u * (tid - (256u - (256u >> L))));
+#pragma unroll
+      for (uint32_t i = 0; i < 128u; i += 32u) {  // its four sectors
+        uint32_t word;
+        asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(word) : "l"(p + i));
+      }
+    }
+    load_cross(ctw, base0, tw);
+    pdl_wait();
     uint32_t v[16];
     if constexpr (DESC) {
       // Distributed shared memory may be written only once every block of the
@@ -113,14 +168,14 @@ struct ClusterNtt {
       for (int gi = 0; gi < GPT; ++gi)
 #pragma unroll
         for (int k = 0; k < G; ++k) v[gi * G + k] = col[base0 + (uint32_t)gi * NT + ((uint32_t)k << 12)];
-      cross(v, base0, tw, 0u, 0u);
+      cross(v, ctw, 0u, 0u);
       asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 #pragma unroll
       for (int gi = 0; gi < GPT; ++gi)
 #pragma unroll
         for (int k = 0; k < G; ++k) {
-          uint32_t* owner = cluster.map_shared_rank(tile, (unsigned)(k >> 1));
-          owner[TP::sw(base0 + (uint32_t)gi * NT + ((uint32_t)(k & 1) << 12))] = v[gi * G + k];
+          uint32_t* owner = cluster.map_shared_rank(tile, (unsigned)k);
+          owner[TP::sw(base0 + (uint32_t)gi * NT)] = v[gi * G + k];
         }
       cluster.sync();  // every block complete (and the staged twiddles visible)
       TP::template ld<TP::kFirst>(tile, v, tid);
@@ -151,14 +206,14 @@ struct ClusterNtt {
       for (int gi = 0; gi < GPT; ++gi)
 #pragma unroll
         for (int k = 0; k < G; ++k) {
-          const uint32_t* owner = cluster.map_shared_rank(tile, (unsigned)(k >> 1));
-          v[gi * G + k] = owner[TP::sw(base0 + (uint32_t)gi * NT + ((uint32_t)(k & 1) << 12))];
+          const uint32_t* owner = cluster.map_shared_rank(tile, (unsigned)k);
+          v[gi * G + k] = owner[TP::sw(base0 + (uint32_t)gi * NT)];
         }
       // No block may leave while another still reads it: arrive once the
       // reads are performed (release), wait only before leaving, so the
       // barrier overlaps the cross layers and the stores.
       asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-      cross(v, base0, tw, scale_w, scale_ws);
+      cross(v, ctw, scale_w, scale_ws);
 #pragma unroll
       for (int gi = 0; gi < GPT; ++gi)
 #pragma unroll
@@ -169,9 +224,8 @@ struct ClusterNtt {
 };
 
 template <class F, bool DESC, int X>
-__global__ void __launch_bounds__(512, 1) cluster_ntt_kernel(uint32_t* d, const uint2* tw, uint32_t scale_w,
-                                                             uint32_t scale_ws) {
-  pdl_enter();
+__global__ void __launch_bounds__(ClusterNtt<F, DESC, X>::NT, 3)
+cluster_ntt_kernel(uint32_t* d, const uint2* tw, uint32_t scale_w, uint32_t scale_ws) {
   ClusterNtt<F, DESC, X>::run(d, tw, scale_w, scale_ws);
 }
 
@@ -179,9 +233,11 @@ template <class F, bool DESC, int X>
 Status launch_cluster(sfntt_ctx* ctx, uint32_t* d, uint32_t batch, const uint2* tw, uint32_t scale_w,
                       cudaStream_t s) {
   using C = ClusterNtt<F, DESC, X>;
-  constexpr int smem = 4 * (int)kTileWords + 8 * (int)C::TP::TW_ENTRIES + 1024;
+  constexpr int smem = 4 * (int)C::TP::TWORDS + 8 * (int)C::TP::TW_ENTRIES + 1024;
   auto kern = cluster_ntt_kernel<F, DESC, X>;
   static std::atomic<uint64_t> smem_done{0};
+  if (C::CS > 8 && !(smem_done.load(std::memory_order_acquire) & (1ull << (ctx->device & 63))))
+    SFNTT_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   SFNTT_TRY(smem_limit_once(kern, smem, ctx->device, smem_done));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(batch * (uint32_t)C::CS);
@@ -193,14 +249,13 @@ Status launch_cluster(sfntt_ctx* ctx, uint32_t* d, uint32_t batch, const uint2* 
   attr[0].val.clusterDim.x = (unsigned)C::CS;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  // small grids: programmatic dependent launch, as the passes do (pdl.cuh)
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
 #ifdef SFNTT_NO_PDL
   cfg.numAttrs = 1;
 #else
-  cfg.numAttrs = pdl_fits(cfg.gridDim.x) ? 2 : 1;
+  cfg.numAttrs = 2;
 #endif
   const uint32_t scale_ws = (uint32_t)(((uint64_t)scale_w << 32) / F::P);
   launch_begin(ctx, s);
@@ -224,10 +279,19 @@ Status cluster_dispatch(sfntt_ctx* ctx, uint32_t* d, uint32_t log_n, uint32_t ba
 
 }  // namespace
 
-bool cluster_ntt_fits(const sfntt_ctx* ctx, uint32_t log_n, uint32_t batch, const void* d) {
+// Against the passes (forward + inverse): BabyBear / KoalaBear win while the
+// blocks fit one wave of three per SM (2^15 x 40 20 against 27 us, 2^14 x 80 19
+// against 22 us; 2^14 x 140 27 against 22 us).  M31's passes over shorter columns
+// read their twiddles from L2 or stage them per tile, so it wins there for far
+// longer (2^14 x 600 75 against 89 us, 2^13 x 1000 59 against 71 us, 2^15 x 290 79
+// against 81 us).  2^16 points keep the line of the 2^13-word blocks, two tiles
+// per SM (x 9 16 against 20 us, x 24 26 against 28 us, M31 26 against 32 us; at the
+// very end, x 37, 36 against 29 us and M31 35 against 32 us).
+bool cluster_ntt_fits(const sfntt_ctx* ctx, int field, uint32_t log_n, uint32_t batch, const void* d) {
   if (ctx->no_cluster || log_n < 13 || log_n > 16 || batch == 0) return false;
   if ((reinterpret_cast<uintptr_t>(d) & 15u) != 0) return false;
-  return ((uint64_t)batch << (log_n - 13)) <= 2ull * (uint64_t)ctx->sm_count;  // one wave
+  const uint64_t waves = log_n == 16 ? 4 : is_monty(field) ? 3 : 16;
+  return ((uint64_t)batch << (log_n - 12)) <= waves * (uint64_t)ctx->sm_count;
 }
 
 Status cluster_ntt_dev(sfntt_ctx* ctx, int field, bool inverse, uint32_t* d, uint32_t log_n, uint32_t batch,

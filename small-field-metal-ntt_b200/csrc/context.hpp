@@ -206,9 +206,9 @@ Status layers_dev(sfntt_ctx* ctx, int field, bool inverse, const uint32_t* in, u
 Status m31_pairs_dev(sfntt_ctx* ctx, bool inverse, uint32_t* d, uint32_t log_n, uint32_t batch, uint32_t scale_w,
                      const uint2* tw, cudaStream_t stream, bool* done);
 // One-launch NTT of 2^13 .. 2^16-point columns on a thread-block cluster
-// (cluster_ntt.cu), in place on dense columns; fits: shape, alignment and at
-// most one wave of CTAs.
-bool cluster_ntt_fits(const sfntt_ctx* ctx, uint32_t log_n, uint32_t batch, const void* d);
+// (cluster_ntt.cu), in place on dense columns; fits: shape, alignment and a
+// batch that the clusters run faster than the passes.
+bool cluster_ntt_fits(const sfntt_ctx* ctx, int field, uint32_t log_n, uint32_t batch, const void* d);
 Status cluster_ntt_dev(sfntt_ctx* ctx, int field, bool inverse, uint32_t* d, uint32_t log_n, uint32_t batch,
                        const uint2* tw, uint32_t scale_w, cudaStream_t stream);
 Status ntt_dev_oop(sfntt_ctx* ctx, int field, bool inverse, const uint32_t* d_in, uint32_t* d_out,

@@ -21,10 +21,13 @@
 
 namespace sfntt {
 
-// First statement of every kernel launched with launch_pdl.
+// First statement of every kernel launched with launch_pdl (or the two halves,
+// with loads of tables -- finished before any launch that uses them -- between).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
 }
 
 // PDL for a grid of `ctas` CTAs.
