@@ -15,12 +15,13 @@ using sfntt::Status;
 
 namespace {
 
-// Restores the caller's current device on scope exit.
+// Restores the caller's current device on scope exit (where it is another one).
 struct DeviceGuard {
   int prev = -1;
   explicit DeviceGuard(int dev) {
     if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
     if (prev != dev) cudaSetDevice(dev);
+    else prev = -1;
   }
   ~DeviceGuard() {
     if (prev >= 0) cudaSetDevice(prev);
@@ -39,7 +40,10 @@ Status device_flag(sfntt_ctx* ctx) {
 }
 
 int finish(sfntt_ctx* ctx, const Status& s) {
-  if (ctx) ctx->last_error = s.ok() ? std::string() : s.msg;
+  if (ctx) {
+    if (s.ok()) ctx->last_error.clear();
+    else ctx->last_error = s.msg;
+  }
   return s.code;
 }
 

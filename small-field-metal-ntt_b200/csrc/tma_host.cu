@@ -12,25 +12,32 @@ namespace {
 // Encoded maps, keyed by every encoding parameter.  A map is a pure function
 // of its key (address, shape, strides, box, swizzle), so an entry never goes
 // stale; repeated launches on the same buffers skip the encoding.
+struct MapKey {
+  uint64_t w[13];  // base, rank and swizzle, dims[5], strides[4], boxes three per word
+  bool operator==(const MapKey& o) const { return std::memcmp(w, o.w, sizeof w) == 0; }
+};
+struct MapHash {
+  size_t operator()(const MapKey& k) const {
+    uint64_t h = 0x9E3779B97F4A7C15ull;
+    for (uint64_t x : k.w) h = (h ^ x) * 0xFF51AFD7ED558CCDull, h ^= h >> 32;
+    return (size_t)h;
+  }
+};
 std::mutex g_map_mu;
-std::unordered_map<std::string, CUtensorMap> g_maps;
+std::unordered_map<MapKey, CUtensorMap, MapHash> g_maps;
 constexpr size_t kMaxMaps = 4096;
 
-std::string map_key(const void* base, uint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
-                    const cuuint32_t* box, bool swizzle128) {
-  struct {
-    const void* base;
-    uint64_t rank_swz;
-    cuuint64_t dims[5], strides[4];
-    cuuint32_t box[5];
-  } k;
+MapKey map_key(const void* base, uint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
+               const cuuint32_t* box, bool swizzle128) {
+  MapKey k;
   std::memset(&k, 0, sizeof k);
-  k.base = base;
-  k.rank_swz = ((uint64_t)rank << 1) | (swizzle128 ? 1u : 0u);
-  std::memcpy(k.dims, dims, rank * sizeof(cuuint64_t));
-  std::memcpy(k.strides, strides_bytes, (rank - 1) * sizeof(cuuint64_t));
-  std::memcpy(k.box, box, rank * sizeof(cuuint32_t));
-  return std::string(reinterpret_cast<const char*>(&k), sizeof k);
+  k.w[0] = reinterpret_cast<uint64_t>(base);
+  k.w[1] = ((uint64_t)rank << 1) | (swizzle128 ? 1u : 0u);
+  for (uint32_t i = 0; i < rank; ++i) k.w[2 + i] = dims[i];
+  for (uint32_t i = 0; i + 1 < rank; ++i) k.w[7 + i] = strides_bytes[i];
+  // boxes are at most 256 per dimension
+  for (uint32_t i = 0; i < rank; ++i) k.w[11 + i / 3] |= (uint64_t)box[i] << (20u * (i % 3));
+  return k;
 }
 
 }  // namespace
@@ -38,7 +45,7 @@ std::string map_key(const void* base, uint32_t rank, const cuuint64_t* dims, con
 Status tensor_map_encode(CUtensorMap* map, const void* base, uint32_t rank, const cuuint64_t* dims,
                          const cuuint64_t* strides_bytes, const cuuint32_t* box, bool swizzle128) {
   if (rank < 1 || rank > 5) return {SFNTT_INVALID_ARGUMENT, "tensor map rank"};
-  const std::string key = map_key(base, rank, dims, strides_bytes, box, swizzle128);
+  const MapKey key = map_key(base, rank, dims, strides_bytes, box, swizzle128);
   {
     std::lock_guard<std::mutex> lk(g_map_mu);
     auto it = g_maps.find(key);

@@ -312,12 +312,16 @@ class NttBackend:
 
     # device pointers (e.g. torch tensors' data_ptr()) on a CUDA stream handle
     def forward_dev(self, ptr: int, log_n: int, batch: int = 1, stream: int = 0) -> None:
-        st = _ffi.lib().sfntt_forward_dev(self.ctx.handle, self.FIELD, self.VARIANT, ptr, log_n, batch, stream)
-        _check(self.ctx.handle, st, batch << log_n)
+        h = self.ctx.handle
+        st = _ffi.lib().sfntt_forward_dev(h, self.FIELD, self.VARIANT, ptr, log_n, batch, stream)
+        if st:
+            _check(h, st, batch << log_n)
 
     def inverse_dev(self, ptr: int, log_n: int, batch: int = 1, stream: int = 0) -> None:
-        st = _ffi.lib().sfntt_inverse_dev(self.ctx.handle, self.FIELD, self.VARIANT, ptr, log_n, batch, stream)
-        _check(self.ctx.handle, st, batch << log_n)
+        h = self.ctx.handle
+        st = _ffi.lib().sfntt_inverse_dev(h, self.FIELD, self.VARIANT, ptr, log_n, batch, stream)
+        if st:
+            _check(h, st, batch << log_n)
 
 
 # M31 Circle NTT (DCCT) variants (src/ntt/m31/*)
