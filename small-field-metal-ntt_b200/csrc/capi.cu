@@ -132,78 +132,112 @@ int api_ntt_gpu(sfntt_ctx* ctx, int field, int variant, bool inverse, const uint
   return finish(ctx, s);
 }
 
+// The context's copier for a download to `dst`; nullptr: copy directly (pinned
+// or registered memory, small copies, or no copier to be had).
+sfntt::HostCopier* copier_for(sfntt_ctx* ctx, const void* dst, size_t bytes) {
+  if (bytes < ((size_t)1 << 20)) return nullptr;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return nullptr;
+  if (!ctx->copier) ctx->copier = sfntt::HostCopier::create(ctx->device);
+  return ctx->copier.get();
+}
+
+// `count` events from a context's pool.
+Status pooled_events(std::vector<cudaEvent_t>& pool, size_t count, unsigned flags) {
+  while (pool.size() < count) {
+    cudaEvent_t e = nullptr;
+    SFNTT_CU(cudaEventCreateWithFlags(&e, flags));
+    pool.push_back(e);
+  }
+  return {};
+}
+
 // Host-memory LDE: columns are processed in chunks on two buffer slots so
 // that the upload of chunk i+1 and the download of chunk i-1 overlap the
 // compute of chunk i.  The download (2^added_bits times the upload) is the
 // bottleneck; chunks grow from an eighth of the slot, doubling, so each
 // upload ends before the previous chunk's download and the download stream
-// starts early and stays busy.
+// starts early and stays busy.  A chunk moves 4 MiB at least: below that its
+// dozen driver calls cost more than the overlap gives.  Outputs in pageable
+// memory leave through the context's copier (host_copy.hpp).  On numpy arrays,
+// before (driver staging, events made per call, an eighth first) -> now: 2^14 x
+// 40 2x 757 -> 367 us, 2^10 x 20 243 -> 78 us, 2^20 x 64 136 -> 70 ms.
 Status run_host_lde(sfntt_ctx* ctx, int field, const uint32_t* in, uint32_t* out, uint32_t log_n, uint32_t batch,
                     uint32_t added_bits, uint32_t shift_monty, int mode, uint64_t* ns) {
   const uint32_t log_ext = log_n + added_bits;
   const size_t n = (size_t)1 << log_n, n_ext = (size_t)1 << log_ext;
   const size_t per_col = (n + n_ext) * sizeof(uint32_t);
   const size_t target = (size_t)192 << 20;  // bytes per slot
-  uint32_t chunk = (uint32_t)std::max<size_t>(1, std::min<size_t>(batch, target / per_col));
+  const size_t least = (size_t)4 << 20;     // bytes per chunk
+  const uint32_t chunk = (uint32_t)std::max<size_t>(1, std::min<size_t>(batch, target / per_col));
+  const uint32_t first = std::max<uint32_t>(std::max<uint32_t>(1, chunk / 8),
+                                            (uint32_t)std::min<size_t>(chunk, (least + per_col - 1) / per_col));
   std::vector<uint32_t> starts;  // first column of each chunk
-  for (uint32_t c0 = 0, size = std::max<uint32_t>(1, chunk / 8); c0 < batch; c0 += size, size = std::min(2 * size, chunk))
-    starts.push_back(c0);
+  for (uint32_t c0 = 0, size = first; c0 < batch; c0 += size, size = std::min(2 * size, chunk)) starts.push_back(c0);
   const uint32_t nchunks = (uint32_t)starts.size();
   SFNTT_TRY(ctx->buf_in.reserve(2 * (size_t)chunk * n * sizeof(uint32_t)));
   SFNTT_TRY(ctx->buf_out.reserve(2 * (size_t)chunk * n_ext * sizeof(uint32_t)));
   uint32_t* din[2] = {ctx->buf_in.as<uint32_t>(), ctx->buf_in.as<uint32_t>() + (size_t)chunk * n};
   uint32_t* dout[2] = {ctx->buf_out.as<uint32_t>(), ctx->buf_out.as<uint32_t>() + (size_t)chunk * n_ext};
 
-  std::vector<cudaEvent_t> evs;
-  auto mk = [&](cudaEvent_t* e, unsigned flags) -> Status {
-    SFNTT_CU(cudaEventCreateWithFlags(e, flags));
-    evs.push_back(*e);
+  SFNTT_TRY(pooled_events(ctx->pipe_events, 6, cudaEventDisableTiming));
+  SFNTT_TRY(pooled_events(ctx->pipe_timers, 2 * (size_t)nchunks, cudaEventDefault));
+  struct Slot { cudaEvent_t uploaded, computed, downloaded; bool used = false; } slot[2];
+  for (int i = 0; i < 2; ++i) {
+    slot[i].uploaded = ctx->pipe_events[3 * i];
+    slot[i].computed = ctx->pipe_events[3 * i + 1];
+    slot[i].downloaded = ctx->pipe_events[3 * i + 2];
+  }
+  cudaEvent_t* t0 = ctx->pipe_timers.data();
+  cudaEvent_t* t1 = t0 + nchunks;
+  cudaStream_t up = ctx->copy_streams[0], down = ctx->copy_streams[1], comp = ctx->stream;
+  sfntt::HostCopier* copier = copier_for(ctx, out, (size_t)batch * n_ext * sizeof(uint32_t));
+  auto cols_of = [&](uint32_t c) { return (c + 1 < nchunks ? starts[c + 1] : batch) - starts[c]; };
+  auto upload_and_compute = [&](uint32_t c) -> Status {
+    Slot& sl = slot[c & 1];
+    const uint32_t cols = cols_of(c);
+    if (sl.used) {
+      SFNTT_CU(cudaStreamWaitEvent(up, sl.computed, 0));      // input slot free
+      SFNTT_CU(cudaStreamWaitEvent(comp, sl.downloaded, 0));  // output slot free
+    }
+    SFNTT_CU(cudaMemcpyAsync(din[c & 1], in + (size_t)starts[c] * n, (size_t)cols * n * 4, cudaMemcpyHostToDevice, up));
+    SFNTT_CU(cudaEventRecord(sl.uploaded, up));
+    SFNTT_CU(cudaStreamWaitEvent(comp, sl.uploaded, 0));
+    SFNTT_CU(cudaEventRecord(t0[c], comp));
+    if (sfntt::is_monty(field))
+      SFNTT_TRY(sfntt::monty_lde_dev(ctx, field, din[c & 1], dout[c & 1], log_n, cols, added_bits, shift_monty, mode, comp));
+    else
+      SFNTT_TRY(sfntt::m31_lde_dev(ctx, din[c & 1], dout[c & 1], log_n, cols, added_bits, comp, mode == kCircleLde));
+    SFNTT_CU(cudaEventRecord(t1[c], comp));
+    SFNTT_CU(cudaEventRecord(sl.computed, comp));
     return {};
   };
-  struct Slot { cudaEvent_t uploaded, computed, downloaded; bool used = false; } slot[2];
-  std::vector<cudaEvent_t> t0(nchunks), t1(nchunks);
+  auto download = [&](uint32_t c) -> Status {
+    Slot& sl = slot[c & 1];
+    const size_t bytes = (size_t)cols_of(c) * n_ext * 4;
+    SFNTT_CU(cudaStreamWaitEvent(down, sl.computed, 0));
+    if (copier) SFNTT_CU(copier->download(out + (size_t)starts[c] * n_ext, dout[c & 1], bytes, down));
+    else SFNTT_CU(cudaMemcpyAsync(out + (size_t)starts[c] * n_ext, dout[c & 1], bytes, cudaMemcpyDeviceToHost, down));
+    SFNTT_CU(cudaEventRecord(sl.downloaded, down));
+    sl.used = true;
+    return {};
+  };
+  // A download into pageable memory holds this thread (the driver stages it
+  // here, or the copier's ring is full), so the next chunk is under way first;
+  // its slot's previous download was issued one step earlier.
   Status st;
-  for (int i = 0; i < 2 && st.ok(); ++i) {
-    st = mk(&slot[i].uploaded, cudaEventDisableTiming);
-    if (st.ok()) st = mk(&slot[i].computed, cudaEventDisableTiming);
-    if (st.ok()) st = mk(&slot[i].downloaded, cudaEventDisableTiming);
-  }
-  for (uint32_t c = 0; c < nchunks && st.ok(); ++c) {
-    st = mk(&t0[c], cudaEventDefault);
-    if (st.ok()) st = mk(&t1[c], cudaEventDefault);
-  }
-  cudaStream_t up = ctx->copy_streams[0], down = ctx->copy_streams[1], comp = ctx->stream;
-  for (uint32_t c = 0; c < nchunks && st.ok(); ++c) {
-    const int k = c & 1;
-    const uint32_t c0 = starts[c];
-    const uint32_t cols = (c + 1 < nchunks ? starts[c + 1] : batch) - c0;
-    auto step = [&]() -> Status {
-      if (slot[k].used) {
-        SFNTT_CU(cudaStreamWaitEvent(up, slot[k].computed, 0));     // input slot free
-        SFNTT_CU(cudaStreamWaitEvent(comp, slot[k].downloaded, 0)); // output slot free
-      }
-      SFNTT_CU(cudaMemcpyAsync(din[k], in + (size_t)c0 * n, (size_t)cols * n * 4, cudaMemcpyHostToDevice, up));
-      SFNTT_CU(cudaEventRecord(slot[k].uploaded, up));
-      SFNTT_CU(cudaStreamWaitEvent(comp, slot[k].uploaded, 0));
-      SFNTT_CU(cudaEventRecord(t0[c], comp));
-      if (sfntt::is_monty(field))
-        SFNTT_TRY(sfntt::monty_lde_dev(ctx, field, din[k], dout[k], log_n, cols, added_bits, shift_monty, mode, comp));
-      else
-        SFNTT_TRY(sfntt::m31_lde_dev(ctx, din[k], dout[k], log_n, cols, added_bits, comp, mode == kCircleLde));
-      SFNTT_CU(cudaEventRecord(t1[c], comp));
-      SFNTT_CU(cudaEventRecord(slot[k].computed, comp));
-      SFNTT_CU(cudaStreamWaitEvent(down, slot[k].computed, 0));
-      SFNTT_CU(cudaMemcpyAsync(out + (size_t)c0 * n_ext, dout[k], (size_t)cols * n_ext * 4, cudaMemcpyDeviceToHost,
-                               down));
-      SFNTT_CU(cudaEventRecord(slot[k].downloaded, down));
-      slot[k].used = true;
-      return {};
-    };
-    st = step();
+  for (uint32_t c = 0; c <= nchunks && st.ok(); ++c) {
+    if (c < nchunks) st = upload_and_compute(c);
+    if (st.ok() && c > 0) st = download(c - 1);
   }
   cudaError_t e1 = cudaStreamSynchronize(down), e2 = cudaStreamSynchronize(comp), e3 = cudaStreamSynchronize(up);
-  if (st.ok() && (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess)) {
-    cudaError_t e = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3);
+  const cudaError_t e4 = copier ? copier->finish() : cudaSuccess;  // on every path: the copier's threads hold `out`
+  if (st.ok() && (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess)) {
+    cudaError_t e = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : (e3 != cudaSuccess ? e3 : e4));
     st = {sfntt::map_cuda_error(e), std::string("LDE pipeline: ") + cudaGetErrorString(e)};
   }
   if (st.ok()) st = device_flag(ctx);
@@ -215,7 +249,6 @@ Status run_host_lde(sfntt_ctx* ctx, int field, const uint32_t* in, uint32_t* out
     }
     *ns = (uint64_t)(total * 1e6);
   }
-  for (cudaEvent_t e : evs) cudaEventDestroy(e);
   return st;
 }
 
@@ -294,6 +327,9 @@ void sfntt_ctx_destroy(sfntt_ctx* ctx) {
     for (auto& m : ctx->m31c_tw)
       for (auto& kv : m) kv.second.release();
     for (auto& kv : ctx->lde_tabs) kv.second.release();
+    ctx->copier.reset();
+    for (cudaEvent_t e : ctx->pipe_events) cudaEventDestroy(e);
+    for (cudaEvent_t e : ctx->pipe_timers) cudaEventDestroy(e);
     ctx->buf_in.release();
     ctx->buf_out.release();
     ctx->buf_aux.release();

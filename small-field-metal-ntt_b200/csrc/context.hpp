@@ -7,12 +7,14 @@
 #include <atomic>
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <tuple>
 #include <vector>
 
 #include "../../include/sfntt.h"
+#include "host_copy.hpp"
 
 namespace sfntt {
 
@@ -108,6 +110,10 @@ struct sfntt_ctx {
 
   // staging for host-memory calls
   sfntt::DevBuf buf_in, buf_out, buf_aux;
+  // downloads into pageable memory (made on the first large one)
+  std::unique_ptr<sfntt::HostCopier> copier;
+  // events of the pipelined host calls, reused
+  std::vector<cudaEvent_t> pipe_events, pipe_timers;
   // base-field planes of CM31 transforms (ext.cu)
   sfntt::DevBuf buf_ext;
   // device int set by a kernel whose bounded wait ran out (SFNTT_TIMEOUT)
