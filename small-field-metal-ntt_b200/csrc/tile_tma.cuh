@@ -342,7 +342,7 @@ struct TPass {
                                                   int beta) {
     using M = RM<KD, P, LT, R, k>;
     const uint32_t cm = M::cm(m);
-    const uint32_t L = a.lo + beta;
+    const uint32_t L = CT ? (uint32_t)beta : a.lo + beta;  // contiguous passes start at layer 0
     if constexpr (kStaged) {
       const uint32_t mask = (1u << beta) - 1u;
       if constexpr (KD == Kind::C) {
@@ -393,7 +393,7 @@ struct TPass {
       for (int jj = 0; jj < r; ++jj) {
         const int j = DESC ? (r - 1 - jj) : jj;
         const uint32_t beta = (uint32_t)(b + j);
-        const uint32_t L = a.lo + beta;
+        const uint32_t L = CT ? (uint32_t)beta : a.lo + beta;  // contiguous passes start at layer 0
         const uint32_t n = 1u << a.log_n;
         uint2 tv[E / 2];
         if constexpr (LSTAGE) {

@@ -44,7 +44,8 @@ def test_passes(ctx, field, log_n, tiles):
     stream = torch.cuda.current_stream().cuda_stream
     names = _names(ctx, lambda: b.forward_dev(d.data_ptr(), log_n, batch, stream))
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert any("warp" in k for k in names) == (tiles >= 3 * sms and log_n > 14), names
+    by_cluster = field == "m31" and log_n == 15  # short M31 columns: one cluster launch
+    assert any("warp" in k for k in names) == (tiles >= 3 * sms and not by_cluster), names
     got = d.cpu().numpy().view(np.uint32)
     cols = sorted({0, batch // 2, batch - 1})
     for c in cols:
