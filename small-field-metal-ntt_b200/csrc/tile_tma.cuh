@@ -563,41 +563,47 @@ struct TPass {
     for (int j = 0; j < R; ++j) cmask |= 1u << mp.mpos[j];
     return sw_support(tmask) & sw_support(cmask);
   }
+  // As byte addresses: the overlap lies in the swizzle bits (word bits 2..4) and
+  // every tile buffer is 1024-byte aligned, so the exclusive or applies to the
+  // thread's whole address and the rest is the access's immediate offset -- one
+  // instruction per address that differs, none to scale and add a base.
   template <int k>
-  __device__ static __forceinline__ uint32_t addr(uint32_t sct, int m) {
+  __device__ static __forceinline__ uint32_t base(const uint32_t* st, uint32_t tid) {
+    static_assert((overlap<k>() & ~0x1Cu) == 0, "slot and thread parts overlap in the swizzle bits alone");
+    return tma::smem_addr(st) + 4u * sw(RM<KD, P, LT, R, k>::ctid(tid));
+  }
+  template <int k>
+  __device__ static __forceinline__ uint32_t addr(uint32_t base, int m) {
     using M = RM<KD, P, LT, R, k>;
     constexpr uint32_t O = overlap<k>();
     const uint32_t scm = sw(M::cm(m));
-    return (sct ^ (scm & O)) + (scm & ~O);
+    return (base ^ (4u * (scm & O))) + 4u * (scm & ~O);
   }
 
   template <int k>
   __device__ static __forceinline__ void ld(const uint32_t* st, uint32_t (&v)[E], uint32_t tid) {
-    using M = RM<KD, P, LT, R, k>;
-    const uint32_t sct = sw(M::ctid(tid));
+    const uint32_t b = base<k>(st, tid);
     if constexpr (vec<k>()) {
 #pragma unroll
       for (int m = 0; m < E; m += 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(st + addr<k>(sct, m));
+        const uint4 q = tma::lds128(addr<k>(b, m));
         v[m] = q.x; v[m + 1] = q.y; v[m + 2] = q.z; v[m + 3] = q.w;
       }
     } else {
 #pragma unroll
-      for (int m = 0; m < E; ++m) v[m] = st[addr<k>(sct, m)];
+      for (int m = 0; m < E; ++m) v[m] = tma::lds32(addr<k>(b, m));
     }
   }
 
   template <int k>
   __device__ static __forceinline__ void st(uint32_t* st, const uint32_t (&v)[E], uint32_t tid) {
-    using M = RM<KD, P, LT, R, k>;
-    const uint32_t sct = sw(M::ctid(tid));
+    const uint32_t b = base<k>(st, tid);
     if constexpr (vec<k>()) {
 #pragma unroll
-      for (int m = 0; m < E; m += 4)
-        *reinterpret_cast<uint4*>(st + addr<k>(sct, m)) = make_uint4(v[m], v[m + 1], v[m + 2], v[m + 3]);
+      for (int m = 0; m < E; m += 4) tma::sts128(addr<k>(b, m), v[m], v[m + 1], v[m + 2], v[m + 3]);
     } else {
 #pragma unroll
-      for (int m = 0; m < E; ++m) st[addr<k>(sct, m)] = v[m];
+      for (int m = 0; m < E; ++m) tma::sts32(addr<k>(b, m), v[m]);
     }
   }
 
