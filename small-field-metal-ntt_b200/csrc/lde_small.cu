@@ -200,7 +200,7 @@ Status launch(sfntt_ctx* ctx, SmallLdeArgs a, bool split, cudaStream_t s) {
     grid.y = y;
   }
   launch_begin(ctx, s);
-  SFNTT_CU(launch_pdl(kern, grid, L::NT, L::kSmemBytes, s, pdl_fits((uint64_t)grid.x * grid.y), a));
+  SFNTT_CU(launch_pdl(kern, grid, L::NT, L::kSmemBytes, s, (uint64_t)grid.x * grid.y <= 16, a));
   static const std::string name = std::string(F::kTag) + "_lde_small_C" + std::to_string(P);
   return launch_check(ctx, name.c_str(), s, ((uint64_t)a.batch << P) * 4u * (1u + (1u << a.log_q)));
 }

@@ -1,18 +1,25 @@
 // pdl.cuh -- programmatic dependent launch between consecutive passes.
 //
 // A pass launched with launch_pdl may be scheduled while the previous kernel
-// on its stream is still running; its threads first let their own dependents
-// launch, then wait (griddepcontrol.wait) until every prerequisite grid has
-// completed and its writes are visible, before touching global memory.  The
-// launch gap between passes disappears; the ordering of their memory effects
-// is that of a plain stream.  A kernel launched without the attribute (or
-// after a non-kernel operation) passes the wait at once.
+// on its stream is still running: once every CTA of that kernel has issued its
+// trigger (or ended), the pass's CTAs take the SM slots that come free, run
+// their prologue (barriers, tensor maps, twiddles staged from tables that no
+// kernel in flight writes) and wait (griddepcontrol.wait) until every
+// prerequisite grid has completed and its writes are visible, before touching
+// data.  The launch gap and the prologue then overlap the previous kernel's
+// end; the ordering of memory effects is that of a plain stream.  A kernel
+// launched without the attribute (or after a non-kernel operation) passes the
+// wait at once.
 //
-// Used for tiny grids only (pdl_fits): there the launch gap is most of a
-// pass's time.  An early-launched grid is placed on whatever SM slots are free
-// while the previous pass still runs; measured on B200, partial grids then
-// end up packed onto part of the GPU and full persistent grids of the
-// four-step BabyBear passes run slower, so larger grids launch plainly.
+// Small kernels trigger at their start; the persistent passes when a CTA starts
+// its last tile.  (Triggered at the start, a next grid waiting in every free slot
+// slowed the full four-step passes by 10 %.)  A persistent grid launched early
+// fills slots in the order they come free, so CTAs with one tile more than others
+// can end up on one SM: pdl_fits takes the grids whose tiles divide evenly and
+// those of eight rounds or more.  Forward + inverse, plain -> early launch:
+// BabyBear 2^20 x 1 24.4 -> 21.4 us, KoalaBear 2^17 x 37 48.0 -> 44.9 us, BabyBear
+// 2^19 x 64 281 -> 274 us, M31 blow-up 2^16 x 100 85 -> 82 us; not taken: 2^24 x 1
+// (6.9 rounds) 209 -> 213 us, CM31 2^16 x 24 (1.3 rounds) 43 -> 46 us.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -30,8 +37,10 @@ __device__ __forceinline__ void pdl_enter() {
   pdl_wait();
 }
 
-// PDL for a grid of `ctas` CTAs.
-inline bool pdl_fits(uint64_t ctas) { return ctas <= 16; }
+// PDL for a grid of `ctas` CTAs over `tiles` tiles.
+inline bool pdl_fits(uint64_t ctas, uint64_t tiles) {
+  return ctas <= 16 || tiles % ctas == 0 || tiles >= 8 * ctas;
+}
 
 template <class... KArgs, class... Args>
 inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl,

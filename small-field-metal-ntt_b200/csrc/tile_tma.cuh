@@ -891,6 +891,7 @@ struct TPass {
       tma::fence_mbar_init();
     }
     __syncthreads();  // staged twiddles and barriers: the halves' last shared step
+    pdl_wait();
     const int32_t hrow = (int32_t)(half * HROWS);
     if (leader) {
       const Geo g0 = geo(a, t);
@@ -905,6 +906,7 @@ struct TPass {
       // tile word c of this half (bit CB-1 = half) sits at view + sw(c) = cur + sw(c mod 2^(CB-1))
       uint32_t* view = cur - half * HWORDS;
       const uint32_t tn = t + t_step;
+      if (tn >= t_end) pdl_trigger();  // the CTA's last tile
       if (leader && tn < t_end) {
         tma::wait_reads();  // the store that last used the other buffer has read it
         const Geo gn = geo(a, tn);
@@ -978,6 +980,7 @@ struct TPass {
       tma::fence_mbar_init();
     }
     __syncthreads();
+    pdl_wait();
     if (tid == 0) {
       for (uint32_t b = 0; b + 1 < NS; ++b) {  // tiles 0 .. NS-2 of this CTA
         const uint32_t tb = t + b * t_step;
@@ -993,6 +996,7 @@ struct TPass {
       const uint32_t buf = it % NS;
       uint32_t* cur = stage + buf * TWORDS;
       const uint32_t tn = t + (NS - 1u) * t_step;  // the tile NS-1 ahead, into the buffer tile it-1 used
+      if (t + t_step >= t_end) pdl_trigger();      // the CTA's last tile
       if (tid == 0 && tn < t_end) {
         const uint32_t nb = (it + NS - 1u) % NS;
         tma::wait_reads();  // the store of tile it-1 (the last one issued) has read that buffer
@@ -1079,7 +1083,6 @@ template <class F, bool DESC, Kind KD, int P, bool PLAIN, bool TW, bool LSTAGE =
 __global__ void __launch_bounds__(TPass<F, DESC, KD, P, PLAIN, TW, LSTAGE, HALVES>::NT,
                                   TPass<F, DESC, KD, P, PLAIN, TW, LSTAGE, HALVES>::kCtasPerSm)
 tma_pass_kernel(const __grid_constant__ CUtensorMap min, const __grid_constant__ CUtensorMap mout, TmaArgs a) {
-  pdl_enter();
   TPass<F, DESC, KD, P, PLAIN, TW, LSTAGE, HALVES>::run(&min, &mout, a);
 }
 
@@ -1309,6 +1312,7 @@ struct TExpand {
       tma::fence_mbar_init();
     }
     __syncthreads();
+    pdl_wait();
     if (tid == 0) {
       tma::mbar_expect_tx(&bar[0], TBYTES);
       Inv::tma_load(min, Inv::geo(ai, t), stage, &bar[0]);
@@ -1318,6 +1322,7 @@ struct TExpand {
       const uint32_t buf = it & 1u;
       uint32_t* cur = stage + buf * TWORDS;
       const uint32_t tn = t + t_step;
+      if (tn >= t_end) pdl_trigger();  // the CTA's last tile
       if (tid == 0) {
         tma::wait_reads();  // every earlier store has read its buffer (tile_body relies on it)
         if (tn < t_end) {
@@ -1414,6 +1419,7 @@ struct TExpandC {
       tma::fence_mbar_init();
     }
     __syncthreads();
+    pdl_wait();
     if (tid == 0) {
       tma::mbar_expect_tx(&bar[0], TBYTES);
       Inv::tma_load(min, Inv::geo(a, t), stage, &bar[0]);
@@ -1425,6 +1431,7 @@ struct TExpandC {
       const uint32_t buf = it & 1u;
       uint32_t* cur = stage + buf * TWORDS;
       const uint32_t tn = t + gridDim.x;
+      if (tn >= a.ntiles) pdl_trigger();  // the CTA's last tile
       if (tid == 0) {
         // The other input buffer was last read by this CTA's previous tile
         // (all threads are past its barriers); ostage, by the previous tile's
@@ -1478,14 +1485,12 @@ struct TExpandC {
 template <class F>
 __global__ void __launch_bounds__(TExpandC<F>::NT, 1)
 tma_expand_c_kernel(const __grid_constant__ CUtensorMap min, const __grid_constant__ CUtensorMap mout, TmaArgs a) {
-  pdl_enter();
   TExpandC<F>::run(&min, &mout, a);
 }
 
 template <class F, int P, bool PLAIN, bool LSTAGE>
 __global__ void __launch_bounds__(TExpand<F, P, PLAIN, LSTAGE>::NT, TExpand<F, P, PLAIN, LSTAGE>::kCtasPerSm)
 tma_expand_kernel(const __grid_constant__ CUtensorMap min, const __grid_constant__ CUtensorMap mout, TmaArgs a) {
-  pdl_enter();
   TExpand<F, P, PLAIN, LSTAGE>::run(&min, &mout, a);
 }
 

@@ -290,6 +290,7 @@ struct WPass {
     }
     wt::fill_table<F>(tab, a.tw, a.log_n, a.lo, 0, tid, wt::kThreads);
     __syncthreads();
+    pdl_wait();
     if (warp == (uint32_t)wt::kWarps) {
       if (lane == 0)
         wt::producer(min, ring, bars, a, 1u, [&](uint32_t it, uint32_t, const uint32_t* src) {
@@ -301,6 +302,7 @@ struct WPass {
     const wt::Lane l(warp, lane);
     uint32_t slot = 0, use = 0;
     for (uint32_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+      if (t + gridDim.x >= a.ntiles) pdl_trigger();  // the CTA's last tile
       uint32_t* buf = ring + slot * kTileWords;
       // A wait that ran out is flagged; the words read then are whatever the
       // buffer holds, and the warp keeps its arrivals.
@@ -328,7 +330,6 @@ struct WPass {
 template <class F, bool DESC>
 __global__ void __launch_bounds__(wt::kThreads, wt::kCtasPerSm)
 warp_pass_kernel(const __grid_constant__ CUtensorMap min, const __grid_constant__ CUtensorMap mout, TmaArgs a) {
-  pdl_enter();
   WPass<F, DESC>::run(&min, &mout, a);
 }
 
@@ -357,6 +358,7 @@ struct WExpandM31 {
     for (uint32_t q = 0; q < nq; ++q)
       wt::fill_table<F>(tabs + (1u + q) * wt::kTabPairs, a.tw_fwd, a.log_n + a.log_q, a.lo, q, tid, wt::kThreads);
     __syncthreads();
+    pdl_wait();
     if (warp == (uint32_t)wt::kWarps) {
       if (lane == 0)
         wt::producer(min, ring, bars, a, nq, [&](uint32_t it, uint32_t q, const uint32_t* src) {
@@ -369,6 +371,7 @@ struct WExpandM31 {
     uint32_t slot = 0, use = 0;    // ring position of the next block
     uint32_t it = 0;
     for (uint32_t t = blockIdx.x; t < a.ntiles; t += gridDim.x, ++it) {
+      if (t + gridDim.x >= a.ntiles) pdl_trigger();  // the CTA's last tile
       if (!tma::mbar_wait(&bars->full[slot], (it / wt::kRing) & 1u, kWaitNs)) atomicExch(a.err, 1);
       __syncwarp();
       uint32_t x[32];
