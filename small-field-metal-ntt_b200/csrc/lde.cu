@@ -186,6 +186,8 @@ Status launch_tma_expand(sfntt_ctx* ctx, const uint32_t* src, uint64_t src_strid
   a.tw = tw_inv;
   a.tw_fwd = tw_fwd;
   a.mul = mul;
+  a.out = d_out;
+  a.out_stride = n_ext;
   a.log_n = log_n;
   a.lo = lo;
   a.batch = batch;
