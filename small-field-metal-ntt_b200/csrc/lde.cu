@@ -211,6 +211,49 @@ Status launch_tma_expand(sfntt_ctx* ctx, const uint32_t* src, uint64_t src_strid
   return launch_check(ctx, name.c_str(), s, ((uint64_t)batch * n) * 4u * (1u + (1u << added_bits)));
 }
 
+// Which staged expansions take two columns at once (TExpandCols): eight or more
+// output blocks -- the one-column form has no registers to load the third and
+// later blocks' multipliers ahead, and waits for each -- on grids whose rounds
+// of column pairs are no more than half the rounds of single columns, plus a
+// twentieth (one CTA per SM in both).  One column -> two, whole LDE 8x: BabyBear
+// 2^20 x 16 738 -> 607 us, 2^19 x 52 1050 -> 942 us, 2^17 x 31 175 -> 157 us, 2^16
+// x 21 73 -> 67 us, KoalaBear 2^18 x 32 16x 645 -> 577 us.  Outside the rule: 2x,
+// where both multipliers are loaded ahead, 2^20 x 256 3.09 -> 3.15 ms; 4x, within
+// 5 % either way (2^17 x 31 102 -> 94 us, 2^21 x 16 809 -> 814 us, 1 % slower beside
+// other kernels); and fewer rounds, 2^16 x 40 8x 118 -> 130 us (3 rounds against 2
+// of twice the work).
+bool expand_cols_fits(const sfntt_ctx* ctx, uint32_t log_n, uint32_t batch, uint32_t added_bits) {
+  const uint64_t sms = (uint64_t)ctx->sm_count, chunks = 1ull << (log_n - 13);
+  const uint64_t pairs = ((batch + 1) / 2 * chunks + sms - 1) / sms, singles = (batch * chunks + sms - 1) / sms;
+  return added_bits >= 3 && 40 * pairs <= 21 * singles;
+}
+
+// The staged expansion of two columns at once, in place in d_out.
+template <class F>
+Status launch_expand_cols(sfntt_ctx* ctx, uint32_t* d_out, uint32_t log_n, uint32_t batch, uint32_t added_bits,
+                          const uint2* tw_inv, const uint2* tw_fwd, const uint2* mul, cudaStream_t s) {
+  using X = TExpandCols<F>;
+  TmaArgs a{};
+  a.tw = tw_inv;
+  a.tw_fwd = tw_fwd;
+  a.mul = mul;
+  a.out = d_out;
+  a.out_stride = 1ull << (log_n + added_bits);
+  a.log_n = log_n;
+  a.lo = log_n - 8;
+  a.batch = batch;
+  a.log_q = added_bits;
+  a.ntiles = ((batch + 1) / 2) << (a.lo - 5);
+  auto kern = tma_expand_cols_kernel<F>;
+  static std::atomic<uint64_t> smem_done{0};
+  SFNTT_TRY(smem_limit_once(kern, (int)X::kSmemBytes, ctx->device, smem_done));
+  const uint32_t grid = std::min<uint32_t>(a.ntiles, (uint32_t)ctx->sm_count);
+  launch_begin(ctx, s);
+  SFNTT_CU(launch_pdl(kern, grid, X::NT, X::kSmemBytes, s, pdl_fits(grid, a.ntiles), a));
+  static const std::string name = std::string(F::kTag) + "_lde_expand_S8cc";
+  return launch_check(ctx, name.c_str(), s, ((uint64_t)batch << log_n) * 4u * (1u + (1u << added_bits)));
+}
+
 // The M31 expansion on warp-owned tiles, up to 4x (each output block's
 // twiddles sit in shared memory) and from three tiles per SM on (tile_warp.cuh).
 __global__ void __launch_bounds__(wt::kThreads, wt::kCtasPerSm)
@@ -371,6 +414,8 @@ Status monty_lde_rows(sfntt_ctx* ctx, const uint32_t* d_in, uint64_t in_stride, 
       if (plain)
         SFNTT_TRY((launch_tma_expand<F, 8, true>(ctx, d_out, n_ext, d_out, log_n, batch, added_bits, tw_inv, tw_fwd,
                                                  mul, s)));
+      else if (batch >= 16 && expand_cols_fits(ctx, log_n, batch, added_bits))
+        SFNTT_TRY((launch_expand_cols<F>(ctx, d_out, log_n, batch, added_bits, tw_inv, tw_fwd, mul, s)));
       else if (batch >= 16)  // the chunk's twiddles are reused across >= 16 columns
         SFNTT_TRY((launch_tma_expand<F, 8, false, true>(ctx, d_out, n_ext, d_out, log_n, batch, added_bits, tw_inv,
                                                         tw_fwd, mul, s)));

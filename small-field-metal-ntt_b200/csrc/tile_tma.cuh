@@ -1405,6 +1405,148 @@ struct TExpand {
   }
 };
 
+// The staged expansion of two columns at once (BabyBear / KoalaBear, 8 layers,
+// eight or more output blocks).  A CTA takes the same 32 positions of columns 2c
+// and 2c + 1, so every twiddle load, multiplier load and address serves two
+// values; the words go between registers and device memory directly (a warp's
+// lanes are 32 consecutive positions, whole 128-byte rows), the next pair's in
+// flight during the last block's forward layers, and shared memory holds the
+// twiddles and one exchange buffer per column.  An odd batch's last column runs
+// alone in its pair.  In place: the first block of every output column is the
+// input.  A warp waits before it writes an exchange until all have read the one
+// before (an mbarrier that each warp arrives on after its reads, so the wait is
+// over by the time a round's layers are done: 2 % of an LDE against a CTA barrier).
+// A row prefetched into L2 a tile ahead changed nothing.  Integer-multiply pipe
+// 62 % busy, 10.2 warp instructions per warp-butterfly (one column: 63 %, 10.5).
+template <class F>
+struct TExpandCols {
+  using X1 = TExpand<F, 8, false, true>;
+  using Inv = typename X1::Inv;
+  using Fwd = typename X1::Fwd;
+  static constexpr int E = X1::E, NT = X1::NT;
+  static constexpr uint32_t TWORDS = X1::TWORDS, TW_ENTRIES = X1::TW_ENTRIES;
+  static constexpr uint32_t kSmemBytes = 2u * X1::TBYTES + 16u * TW_ENTRIES + 16u;
+  using M0 = RM<Kind::S, 8, X1::LT, X1::R, 0>;
+  using M1 = RM<Kind::S, 8, X1::LT, X1::R, 1>;
+  static_assert(X1::K == 2 && M0::cm(1) == 32u && M0::cm(15) == 15u * 32u, "round 0: slot m is element m of the thread's 16");
+
+  __device__ static __forceinline__ void load(uint32_t (&x)[E], const char* p, uint32_t off, uint32_t step) {
+#pragma unroll
+    for (int m = 0; m < E; ++m, off += step) x[m] = *reinterpret_cast<const uint32_t*>(p + off);
+  }
+  __device__ static __forceinline__ void store(const uint32_t (&v)[E], char* p, uint32_t off, uint32_t step) {
+#pragma unroll
+    for (int m = 0; m < E; ++m, off += step) *reinterpret_cast<uint32_t*>(p + off) = v[m];
+  }
+
+  __device__ static void run(const TmaArgs& a) {
+    extern __shared__ __align__(1024) uint32_t smem_words[];
+    uint32_t* bufa = smem_words;
+    uint32_t* bufb = smem_words + TWORDS;
+    uint2* tws_inv = reinterpret_cast<uint2*>(smem_words + 2 * TWORDS);
+    uint2* tws_fwd = tws_inv + TW_ENTRIES;
+    uint64_t* rd = reinterpret_cast<uint64_t*>(tws_fwd + TW_ENTRIES);  // a phase: every warp has read an exchange
+    const uint32_t tid = threadIdx.x;
+    const uint32_t per = (a.ntiles + gridDim.x - 1) / gridDim.x;
+    uint32_t t = blockIdx.x * per;
+    const uint32_t t_end = (t + per < a.ntiles) ? t + per : a.ntiles;
+    if (t >= t_end) return;
+    if (tid == 0) {
+      tma::mbar_init(rd, NT / 32);
+      tma::fence_mbar_init();
+    }
+    uint32_t phase = 0;
+    bool ok = true;
+    const auto has_read = [&] {
+      __syncwarp();
+      if ((tid & 31u) == 0) tma::mbar_arrive(rd);
+    };
+    const auto all_read = [&] {
+      ok &= tma::mbar_wait(rd, phase & 1u, kWaitNs);
+      ++phase;
+    };
+    __syncthreads();
+    has_read();
+    const uint32_t np = (a.batch + 1) / 2;  // column pairs
+    uint32_t chunk = t / np, pair = t % np;
+    const uint32_t n = 1u << a.log_n, nq = 1u << a.log_q;
+    const uint32_t ct0 = M0::ctid(tid), ct1 = M1::ctid(tid);
+    const uint32_t step = 4u << a.lo;
+    const uint32_t off = 4u * ((ct0 & 31u) + ((ct0 >> 5) << a.lo));
+    const uint64_t col_bytes = 4ull * a.out_stride;
+    const typename Inv::Geo gi{};  // per-position twiddles: nothing of the tile's place enters
+    const FwdArgs af = fwd_args(a);
+    pdl_wait();
+    char* pa = reinterpret_cast<char*>(a.out) + (uint64_t)(2 * pair) * col_bytes + 128u * chunk;
+    bool two = 2 * pair + 1 < a.batch;
+    uint32_t xa[E], xb[E];
+    load(xa, pa, off, step);
+    load(xb, two ? pa + col_bytes : pa, off, step);
+    uint32_t staged = ~0u;
+    for (; t < t_end; ++t) {
+      const bool last = t + 1 >= t_end;
+      if (last) pdl_trigger();
+      if (chunk != staged) {
+        __syncthreads();  // the previous pair's twiddle reads
+        Inv::stage_lchunk(tws_inv, a.tw, a.lo, chunk, tid);
+        Fwd::stage_lchunk(tws_fwd, a.tw_fwd, a.lo, chunk, tid);
+        staged = chunk;
+        __syncthreads();
+      }
+      const uint2* mt = a.mul + (chunk << kTileBits) + ct1;
+      Inv::template round2<0>(xa, xb, a, tws_inv, gi, tid);
+      all_read();
+      Inv::template st<0>(bufa, xa, tid);
+      Inv::template st<0>(bufb, xb, tid);
+      uint2 w[E];
+      X1::load_mul(w, mt);
+      __syncthreads();
+      Inv::template ld<1>(bufa, xa, tid);
+      Inv::template ld<1>(bufb, xb, tid);
+      has_read();
+      Inv::template round2<1>(xa, xb, a, tws_inv, gi, tid);
+      char* oa = pa;
+      const bool two_now = two;
+      if (!last) {
+        if (++pair == np) { pair = 0; ++chunk; }
+        pa = reinterpret_cast<char*>(a.out) + (uint64_t)(2 * pair) * col_bytes + 128u * chunk;
+        two = 2 * pair + 1 < a.batch;
+      }
+      for (uint32_t q = 0; q < nq; ++q, oa += 4ull * n) {
+        uint32_t va[E], vb[E];
+#pragma unroll
+        for (int m = 0; m < E; ++m) {
+          va[m] = mul_shoup<F>(xa[m], w[m].x, w[m].y);
+          vb[m] = mul_shoup<F>(xb[m], w[m].x, w[m].y);
+        }
+        Fwd::template round2<1>(va, vb, af, tws_fwd, gi, tid);
+        all_read();
+        Fwd::template st<1>(bufa, va, tid);
+        Fwd::template st<1>(bufb, vb, tid);
+        if (q + 1 < nq) {
+          X1::load_mul(w, mt + (uint64_t)(q + 1) * n);
+        } else if (!last) {
+          load(xa, pa, off, step);
+          load(xb, two ? pa + col_bytes : pa, off, step);
+        }
+        __syncthreads();
+        Fwd::template ld<0>(bufa, va, tid);
+        Fwd::template ld<0>(bufb, vb, tid);
+        has_read();
+        Fwd::template round2<0>(va, vb, af, tws_fwd, gi, tid);
+        store(va, oa, off, step);
+        if (two_now) store(vb, oa + col_bytes, off, step);
+      }
+    }
+    if (!ok) atomicExch(a.err, 1);
+  }
+};
+
+template <class F>
+__global__ void __launch_bounds__(TExpandCols<F>::NT, 1) tma_expand_cols_kernel(TmaArgs a) {
+  TExpandCols<F>::run(a);
+}
+
 // Natural-order LDE expansion (BabyBear / KoalaBear, 2x), the mirror image of
 // TExpand for natural-order input and output rows.  The strided pass before it
 // ran the inverse GS-DIF layers [12, log n) on the natural-order evaluations;
