@@ -297,10 +297,10 @@ Status launch_tma_expand_c(sfntt_ctx* ctx, const uint32_t* src, uint32_t* d_out,
                            const uint2* tw_inv, const uint2* tw_fwd, const uint2* mul, cudaStream_t s) {
   using X = TExpandC<F>;
   const uint64_t n = 1ull << log_n;
-  CUtensorMap min, mout;
+  CUtensorMap min;
   SFNTT_TRY(encode_c_map(&min, src, log_n, n, batch, 12));
-  SFNTT_TRY(encode_c_map(&mout, d_out, log_n + 1, 2 * n, batch, 12));
   TmaArgs a{};
+  a.out = d_out;
   a.tw = tw_inv;
   a.tw_fwd = tw_fwd;
   a.mul = mul;
@@ -312,13 +312,12 @@ Status launch_tma_expand_c(sfntt_ctx* ctx, const uint32_t* src, uint32_t* d_out,
   a.spans = 0;
   a.log_tpc = log_n - kTileBits;
   a.ntiles = (uint32_t)(((uint64_t)batch * n) >> kTileBits);
-  constexpr int smem = 4 * (int)X::TBYTES + 16 + 16 * (int)X::TW_ENTRIES + 1024;
   auto kern = tma_expand_c_kernel<F>;
   static std::atomic<uint64_t> smem_done{0};
-  SFNTT_TRY(smem_limit_once(kern, smem, ctx->device, smem_done));
+  SFNTT_TRY(smem_limit_once(kern, (int)X::kSmemBytes, ctx->device, smem_done));
   const uint32_t grid = std::min<uint32_t>(a.ntiles, (uint32_t)ctx->sm_count);
   launch_begin(ctx, s);
-  SFNTT_CU(launch_pdl(kern, grid, X::NT, smem, s, pdl_fits(grid, a.ntiles), min, mout, a));
+  SFNTT_CU(launch_pdl(kern, grid, X::NT, X::kSmemBytes, s, pdl_fits(grid, a.ntiles), min, a));
   static const std::string name = std::string(F::kTag) + "_lde_expand_tma_C12n";
   return launch_check(ctx, name.c_str(), s, ((uint64_t)batch * n) * 4u * 3u);
 }

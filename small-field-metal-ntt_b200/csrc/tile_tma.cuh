@@ -1363,6 +1363,7 @@ struct TExpand {
       if (tn >= t_end) pdl_trigger();  // the CTA's last tile
       auto load_next = [&] {
         if (tid == 0 && tn < t_end) {
+          if (direct) tma::fence_proxy_async();  // that buffer's exchanges, behind the barrier, come before the load
           tma::mbar_expect_tx(&bar[buf ^ 1u], TBYTES);
           Inv::tma_load(min, Inv::geo(ai, tn), stage + (buf ^ 1u) * TWORDS, &bar[buf ^ 1u]);
         }
@@ -1555,11 +1556,19 @@ __global__ void __launch_bounds__(TExpandCols<F>::NT, 1) tma_expand_cols_kernel(
 // then for each coset r in {0, 1}: multiplies by M_r[p] = n^-1 (shift
 // g_ext^r)^rev(p) and runs the forward CT-DIT layers [0, 12) of the n-point
 // network (forward table).  Coset r's word p belongs at extended position
-// 2p + r, so both cosets are interleaved in shared memory and the tile leaves
-// as 2^14 contiguous words; the strided pass after it runs the DIT layers
-// [12, log n) of every coset on the interleaved column.  The inverse ends and
-// the forward starts in round 0's layout, so the coefficients stay in
-// registers.
+// 2p + r; the strided pass after it runs the DIT layers [12, log n) of every
+// coset on the interleaved column.  The inverse ends and the forward starts in
+// round 0's layout, so the coefficients stay in registers.
+//
+// Bound by the integer pipes: 18 layers' butterflies per word against 12 bytes.
+// One CTA per SM (64 KiB of twiddles) whose two 256-thread halves take the two
+// halves of a tile and never wait for one another.  An exchange is written
+// where the thread read last, so the only barriers are the 256-thread ones
+// inside the exchanges: coset 1 exchanges in a buffer of its own, and both
+// cosets leave straight from registers, 8 bytes per lane, 256 contiguous bytes
+// per warp.  Against whole tiles interleaved in shared memory and stored by TMA
+// (3 to 4 CTA barriers each): BabyBear 2^18 x 100 214 -> 192 us, the natural-order
+// LDE of 2^20 x 256 3.68 -> 3.48 ms.
 template <class F>
 struct TExpandC {
   using Inv = TPass<F, true, Kind::C, 12>;
@@ -1580,103 +1589,95 @@ struct TExpandC {
     for (int m = 0; m < E; ++m) w[m] = __ldg(mq + (uint32_t)m * NT + tid);
   }
 
-  // coset r's values (round K-1 layout, canonical) to the interleaved output tile
-  __device__ static __forceinline__ void put(uint32_t* ostage, const uint32_t (&v)[E], uint32_t ctl, uint32_t r) {
-#pragma unroll
-    for (int m = 0; m < E; ++m) {
-      const uint32_t e = ((ctl | ML::cm(m)) << 1) | r;  // 14-bit extended word of the tile
-      ostage[(e >> 13) * TWORDS + Inv::sw(e & (TWORDS - 1u))] = v[m];
-    }
-  }
+  static constexpr uint32_t HWORDS = TWORDS / 2, HBYTES = TBYTES / 2, HROWS = HWORDS / 32;
+  static constexpr uint32_t kSmemBytes = 3u * TBYTES + 64u + 16u * TW_ENTRIES;
+  static_assert(Inv::halves_ok() && Fwd::halves_ok() && Inv::xgroups(2, 1) == 2 && Fwd::xgroups(1, 2) == 2,
+                "independent halves, each with one barrier of its 256 threads per transform");
+  static_assert(ML::cm(1) == 256u && ML::cm(15) == 15u * 256u, "last round: slot m is tile bits 8..11");
 
-  __device__ static void run(const CUtensorMap* min, const CUtensorMap* mout, const TmaArgs& args) {
+  __device__ static void run(const CUtensorMap* min, const TmaArgs& args) {
     extern __shared__ __align__(1024) uint32_t smem_words[];
-    uint32_t* stage = smem_words;           // 2 x TWORDS: input tiles (double-buffered)
-    uint32_t* ostage = stage + 2 * TWORDS;  // 2 x TWORDS: the tile's two output halves
-    uint64_t* bar = reinterpret_cast<uint64_t*>(ostage + 2 * TWORDS);
-    uint2* tws_inv = reinterpret_cast<uint2*>(bar + 2);
-    uint2* tws_fwd = tws_inv + TW_ENTRIES;
     const uint32_t tid = threadIdx.x;
+    const uint32_t half = tid >> 8;
+    const bool leader = (tid & 255u) == 0u;
+    uint32_t* stage = smem_words + half * 3u * HWORDS;  // two input half tiles, coset 1's exchanges
+    uint32_t* alt = stage + 2u * HWORDS - half * HWORDS;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_words + 3 * TWORDS);
+    uint64_t* bar = bars + 2u * half;
+    volatile uint32_t* bad = reinterpret_cast<uint32_t*>(bars + 4) + half;  // a wait of this half ran out
+    uint2* tws_inv = reinterpret_cast<uint2*>(bars + 8);
+    uint2* tws_fwd = tws_inv + TW_ENTRIES;
     const TmaArgs& a = args;
     uint32_t t = blockIdx.x;
     if (t >= a.ntiles) return;
     Inv::stage_twiddles(tws_inv, a.tw, tid);
     Fwd::stage_twiddles(tws_fwd, a.tw_fwd, tid);
-    if (tid == 0) {
+    if (leader) {
       tma::prefetch_map(min);
-      tma::prefetch_map(mout);
       tma::mbar_init(&bar[0], 1);
       tma::mbar_init(&bar[1], 1);
       tma::fence_mbar_init();
+      *bad = 0u;
     }
-    __syncthreads();
+    __syncthreads();  // the halves' last shared step
     pdl_wait();
-    if (tid == 0) {
-      tma::mbar_expect_tx(&bar[0], TBYTES);
-      Inv::tma_load(min, Inv::geo(a, t), stage, &bar[0]);
+    const int32_t hrow = (int32_t)(half * HROWS);
+    if (leader) {
+      const typename Inv::Geo g0 = Inv::geo(a, t);
+      tma::mbar_expect_tx(&bar[0], HBYTES);
+      Inv::c_load(min, g0.c1 + hrow, g0.c2, stage, &bar[0], false);
     }
     const uint32_t ctl = ML::ctid(tid);
     const uint64_t n = 1ull << a.log_n;
     uint32_t x[E], v[E];
     for (uint32_t it = 0; t < a.ntiles; t += gridDim.x, ++it) {
       const uint32_t buf = it & 1u;
-      uint32_t* cur = stage + buf * TWORDS;
+      uint32_t* view = stage + buf * HWORDS - half * HWORDS;
       const uint32_t tn = t + gridDim.x;
       if (tn >= a.ntiles) pdl_trigger();  // the CTA's last tile
-      if (tid == 0) {
-        // The other input buffer was last read by this CTA's previous tile
-        // (all threads are past its barriers); ostage, by the previous tile's
-        // stores: wait for them here, the barrier before this tile's first
-        // ostage write publishes it.
-        tma::wait_reads();
-        if (tn < a.ntiles) {
-          tma::mbar_expect_tx(&bar[buf ^ 1u], TBYTES);
-          Inv::tma_load(min, Inv::geo(a, tn), stage + (buf ^ 1u) * TWORDS, &bar[buf ^ 1u]);
-        }
+      if (leader && tn < a.ntiles) {
+        // The other buffer was last touched by coset 0 of the previous tile,
+        // before the barrier in coset 1's exchanges.
+        const typename Inv::Geo gn = Inv::geo(a, tn);
+        tma::fence_proxy_async();
+        tma::mbar_expect_tx(&bar[buf ^ 1u], HBYTES);
+        Inv::c_load(min, gn.c1 + hrow, gn.c2, stage + (buf ^ 1u) * HWORDS, &bar[buf ^ 1u], false);
       }
-      const bool ok = tma::mbar_wait(&bar[buf], (it >> 1) & 1u, kWaitNs);
+      if (!tma::mbar_wait(&bar[buf], (it >> 1) & 1u, kWaitNs)) *bad = 1u;
       const typename Inv::Geo g = Inv::geo(a, t);
       uint2 w[E];
       load_mul(w, a.mul + g.pos_base, tid);  // coset 0's, in flight during the inverse layers
-      Inv::template ld<Inv::kFirst>(cur, x, tid);
-      Inv::template rounds<0>(cur, x, a, tws_inv, g, tid);  // x: round 0 layout, canonical
-#pragma unroll
-      for (uint32_t r = 0; r < 2; ++r) {
-#pragma unroll
-        for (int m = 0; m < E; ++m) v[m] = mul_shoup<F>(x[m], w[m].x, w[m].y);
-        if (r == 0) load_mul(w, a.mul + n + g.pos_base, tid);  // coset 1's, during coset 0's layers
-        Fwd::template rounds<0>(cur, v, a, tws_fwd, g, tid);
-#pragma unroll
-        for (int m = 0; m < E; ++m) v[m] = reduce2p<F>(v[m]);  // lazy CT values to [0, p)
-        // coset 0: every thread is done exchanging through cur before coset 1
-        // reuses it, and ostage is free (thread 0 waited at the tile start)
-        if (r == 0) __syncthreads();
-        put(ostage, v, ctl, r);
-      }
-      tma::fence_proxy_async();
-      if (__syncthreads_or(!ok)) {
-        if (tid == 0) {
+      Inv::template ld<Inv::kFirst>(view, x, tid);
+      Inv::template rounds<0>(view, x, a, tws_inv, g, tid);  // x: round 0 layout, canonical
+      // Set before the inverse layers' barrier, read before the next one: the
+      // half's threads agree.
+      if (*bad) {
+        if (leader) {
           atomicExch(a.err, 1);
           if (tn < a.ntiles) tma::mbar_wait(&bar[buf ^ 1u], ((it + 1) >> 1) & 1u, kWaitNs);
-          tma::wait_all();
         }
         return;
       }
-      if (tid == 0) {
-        // extended rows [2 * pos_base, 2 * pos_base + 2^14) of the column, two boxes of 2^13 words
-        Inv::c_store(mout, 2 * g.c1, g.c2, ostage, true);
-        Inv::c_store(mout, 2 * g.c1 + (int32_t)(TWORDS / 32), g.c2, ostage + TWORDS, true);
-        tma::commit();
-      }
+#pragma unroll
+      for (int m = 0; m < E; ++m) v[m] = mul_shoup<F>(x[m], w[m].x, w[m].y);
+      load_mul(w, a.mul + n + g.pos_base, tid);  // coset 1's, during coset 0's layers
+      Fwd::template rounds<0>(view, v, a, tws_fwd, g, tid);
+#pragma unroll
+      for (int m = 0; m < E; ++m) x[m] = mul_shoup<F>(x[m], w[m].x, w[m].y);
+      // alt: its last readers (the previous tile's coset 1) are behind two barriers
+      Fwd::template rounds<0>(alt, x, a, tws_fwd, g, tid);
+      // extended words 2p, 2p + 1 of the column; 256 contiguous bytes per warp
+      uint2* o = reinterpret_cast<uint2*>(a.out + 2ull * n * (uint32_t)g.c2) + g.pos_base + ctl;
+#pragma unroll
+      for (int m = 0; m < E; ++m) o[ML::cm(m)] = make_uint2(reduce2p<F>(v[m]), reduce2p<F>(x[m]));  // lazy CT values to [0, p)
     }
-    if (tid == 0) tma::wait_all();
   }
 };
 
 template <class F>
 __global__ void __launch_bounds__(TExpandC<F>::NT, 1)
-tma_expand_c_kernel(const __grid_constant__ CUtensorMap min, const __grid_constant__ CUtensorMap mout, TmaArgs a) {
-  TExpandC<F>::run(&min, &mout, a);
+tma_expand_c_kernel(const __grid_constant__ CUtensorMap min, TmaArgs a) {
+  TExpandC<F>::run(&min, a);
 }
 
 template <class F, int P, bool PLAIN, bool LSTAGE>

@@ -51,3 +51,38 @@ def test_expansion(ctx, field, log_n, batch, added, two):
     assert any(k.endswith("S8cc") for k in names) == two, names
     if not two:
         assert any("_expand_tma_S8" in k for k in names), names
+
+
+def _rev(k):
+    i = np.arange(1 << k)
+    r = np.zeros_like(i)
+    for _ in range(k):
+        r, i = (r << 1) | (i & 1), i >> 1
+    return r
+
+
+@pytest.mark.parametrize("log_n,batch", [(13, 1), (13, 2), (13, 149), (14, 37), (14, 149), (15, 3), (16, 55), (18, 5), (20, 2)])
+@pytest.mark.parametrize("field", ["bb", "kb"])
+def test_natural_order(ctx, field, log_n, batch):
+    """Natural-order 2x expansion: one tile, one tile per CTA and one more, several per CTA."""
+    p = O.KB_P if field == "kb" else O.BB_P
+    x = O.lcg(batch << log_n, 53 + log_n, p, monty=True)
+    x[::89] = p - 1
+    shift = 999 if batch & 1 else 0
+    br = np.ascontiguousarray(x.reshape(batch, -1)[:, _rev(log_n)]).reshape(-1)
+    ref = (O.kb_coset_lde if field == "kb" else O.bb_coset_lde)(br, log_n, batch, 1, shift_monty=shift, threads=8)
+    ref = ref.reshape(batch, -1)[:, _rev(log_n + 1)].reshape(-1)
+    lde = (sfntt.KbCosetLdeBatch if field == "kb" else sfntt.CosetLdeBatch)(ctx, natural=True)
+    d_in = torch.from_numpy(x.view(np.int32).copy()).cuda()
+    out = torch.full(((batch << (log_n + 1)) + 64,), 99, dtype=torch.int32, device="cuda")
+    ctx.kernel_timing(True)
+    for _ in range(2):
+        out[:-64].fill_(-1)
+        lde.execute_dev(d_in.data_ptr(), out.data_ptr(), log_n, batch, 1, shift_monty=shift,
+                        stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert (out[-64:] == 99).all()
+        assert np.array_equal(out[:-64].cpu().numpy().view(np.uint32), ref)
+    names = list(ctx.kernel_times())
+    ctx.kernel_timing(False)
+    assert log_n == 13 or any(k.endswith("_lde_expand_tma_C12n") for k in names), names
