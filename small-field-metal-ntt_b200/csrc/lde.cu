@@ -204,7 +204,7 @@ Status launch_tma_expand(sfntt_ctx* ctx, const uint32_t* src, uint64_t src_strid
       ctx->tma_ctas > 0 ? std::min<uint32_t>((uint32_t)ctx->tma_ctas, (uint32_t)X::kCtasPerSm) : (uint32_t)X::kCtasPerSm;
   const uint32_t grid = std::min<uint32_t>(a.ntiles, ctas * (uint32_t)ctx->sm_count);
   launch_begin(ctx, s);
-  SFNTT_CU(launch_pdl(kern, grid, X::NT, smem, s, pdl_fits(grid, a.ntiles), min, mout, a));
+  SFNTT_CU(launch_pdl(kern, grid, X::NT, smem, s, pdl_fits_expand(grid, a.ntiles, (uint64_t)ctas * ctx->sm_count, log_n + added_bits), min, mout, a));
   static const std::string name =
       std::string(F::kTag) + "_lde_expand_tma_S" + std::to_string(P) + (PLAIN ? "p" : "") +
       (LSTAGE ? "c" : "");
@@ -249,7 +249,7 @@ Status launch_expand_cols(sfntt_ctx* ctx, uint32_t* d_out, uint32_t log_n, uint3
   SFNTT_TRY(smem_limit_once(kern, (int)X::kSmemBytes, ctx->device, smem_done));
   const uint32_t grid = std::min<uint32_t>(a.ntiles, (uint32_t)ctx->sm_count);
   launch_begin(ctx, s);
-  SFNTT_CU(launch_pdl(kern, grid, X::NT, X::kSmemBytes, s, pdl_fits(grid, a.ntiles), a));
+  SFNTT_CU(launch_pdl(kern, grid, X::NT, X::kSmemBytes, s, pdl_fits_expand(grid, a.ntiles, ctx->sm_count, log_n + added_bits), a));
   static const std::string name = std::string(F::kTag) + "_lde_expand_S8cc";
   return launch_check(ctx, name.c_str(), s, ((uint64_t)batch << log_n) * 4u * (1u + (1u << added_bits)));
 }
@@ -285,7 +285,7 @@ Status launch_warp_expand_m31(sfntt_ctx* ctx, uint32_t* d_out, uint32_t log_n, u
   const uint32_t ctas = ctx->tma_ctas > 0 ? std::min<uint32_t>((uint32_t)ctx->tma_ctas, wt::kCtasPerSm) : wt::kCtasPerSm;
   const uint32_t grid = std::min<uint32_t>(a.ntiles, ctas * (uint32_t)ctx->sm_count);
   launch_begin(ctx, s);
-  SFNTT_CU(launch_pdl(warp_expand_m31_kernel, grid, wt::kThreads, X::kSmemBytes, s, pdl_fits(grid, a.ntiles), min, mout, a));
+  SFNTT_CU(launch_pdl(warp_expand_m31_kernel, grid, wt::kThreads, X::kSmemBytes, s, pdl_fits_expand(grid, a.ntiles, (uint64_t)ctas * ctx->sm_count, log_n + added_bits), min, mout, a));
   return launch_check(ctx, "m31_lde_expand_warp_S8", s, ((uint64_t)batch * n) * 4u * (1u + (1u << added_bits)));
 }
 
@@ -317,7 +317,7 @@ Status launch_tma_expand_c(sfntt_ctx* ctx, const uint32_t* src, uint32_t* d_out,
   SFNTT_TRY(smem_limit_once(kern, (int)X::kSmemBytes, ctx->device, smem_done));
   const uint32_t grid = std::min<uint32_t>(a.ntiles, (uint32_t)ctx->sm_count);
   launch_begin(ctx, s);
-  SFNTT_CU(launch_pdl(kern, grid, X::NT, X::kSmemBytes, s, pdl_fits(grid, a.ntiles), min, a));
+  SFNTT_CU(launch_pdl(kern, grid, X::NT, X::kSmemBytes, s, pdl_fits_expand(grid, a.ntiles, ctx->sm_count, log_n + 1), min, a));
   static const std::string name = std::string(F::kTag) + "_lde_expand_tma_C12n";
   return launch_check(ctx, name.c_str(), s, ((uint64_t)batch * n) * 4u * 3u);
 }

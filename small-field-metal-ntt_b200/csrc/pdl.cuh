@@ -37,9 +37,18 @@ __device__ __forceinline__ void pdl_enter() {
   pdl_wait();
 }
 
-// PDL for a grid of `ctas` CTAs over `tiles` tiles.
-inline bool pdl_fits(uint64_t ctas, uint64_t tiles) {
-  return ctas <= 16 || tiles % ctas == 0 || tiles >= 8 * ctas;
+// PDL for a grid of `ctas` CTAs over `tiles` tiles of columns of 2^log_n words.
+// Not from 2^22 words on: there an early launch gains nothing and mostly loses
+// (plain -> early: BabyBear LDE 2^22 x 64 3.75 -> 3.93 ms, 2^23 x 4 626 -> 668 us,
+// 2^21 x 8, whose output has 2^22, 280 -> 295 us, 2^23 x 9 forward 424 -> 438 us).
+inline bool pdl_fits(uint64_t ctas, uint64_t tiles, uint32_t log_n) {
+  return log_n < 22 && (ctas <= 16 || tiles % ctas == 0 || tiles >= 8 * ctas);
+}
+
+// An expansion of fewer tiles than `slots` (CTAs that fit the GPU) launched early
+// packs onto the SMs that come free first: M31 2^16 x 12 4x 28.6 -> 38.5 us.
+inline bool pdl_fits_expand(uint64_t ctas, uint64_t tiles, uint64_t slots, uint32_t log_n) {
+  return (ctas <= 16 || ctas == slots) && pdl_fits(ctas, tiles, log_n);
 }
 
 template <class... KArgs, class... Args>

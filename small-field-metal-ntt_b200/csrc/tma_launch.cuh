@@ -144,7 +144,7 @@ Status launch_warp_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
   const uint32_t ctas = ctx->tma_ctas > 0 ? std::min<uint32_t>((uint32_t)ctx->tma_ctas, wt::kCtasPerSm) : wt::kCtasPerSm;
   const uint32_t grid = std::min<uint32_t>(a.ntiles, ctas * (uint32_t)ctx->sm_count);
   launch_begin(ctx, s);
-  SFNTT_CU(launch_pdl(kern, grid, wt::kThreads, W::kSmemBytes, s, pdl_fits(grid, a.ntiles), min, mout, a));
+  SFNTT_CU(launch_pdl(kern, grid, wt::kThreads, W::kSmemBytes, s, pdl_fits(grid, a.ntiles, a.log_n), min, mout, a));
   static const std::string name = std::string(F::kTag) + (DESC ? "_fwd" : "_inv") + "_warp_S8" + (F::kMontgomery ? "p" : "");
   return launch_check(ctx, name.c_str(), s, ((uint64_t)r.batch << log_w) * 8u);
 }
@@ -201,7 +201,7 @@ Status launch_tma_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
   const uint32_t grid = std::min<uint32_t>(a.ntiles, ctas * (uint32_t)ctx->sm_count);
   launch_begin(ctx, s);
   // (LSTAGE: contiguous ranges of tiles per CTA, where an early launch gained nothing)
-  SFNTT_CU(launch_pdl(kern, grid, T::NT, smem, s, LSTAGE ? grid <= 16 : pdl_fits(grid, a.ntiles), min, mout, a));
+  SFNTT_CU(launch_pdl(kern, grid, T::NT, smem, s, LSTAGE ? grid <= 16 : pdl_fits(grid, a.ntiles, a.log_n), min, mout, a));
   return launch_check(ctx, tma_pass_name<F, DESC, KD, P, PLAIN, TW, LSTAGE>(), s,
                       ((uint64_t)r.batch << log_w) * 8u);
 }
