@@ -1119,8 +1119,11 @@ struct TExpand {
   // and loads each multiplier where it is used, so it too fits 64 registers
   // and two CTAs per SM.
   static constexpr int kCtasPerSm = (F::kMontgomery && !PLAIN) ? 1 : 2;
-  // Paired blocks stored straight from registers (tile_body_pairs).
-  static constexpr bool kDirect = F::kMontgomery && K == 2 && !PLAIN;
+  // Paired blocks stored straight from registers (tile_body_pairs).  Not where the
+  // twiddles come from memory: those loads wait behind the stores (direct -> TMA
+  // store: LDE 2^20 x 8 2x 136 -> 128 us, 2^22 x 8 561 -> 530 us, 2^24 x 5 1510 ->
+  // 1422 us; one tile per CTA, 2^20 x 1, 25.3 -> 25.9 us).
+  static constexpr bool kDirect = F::kMontgomery && K == 2 && !PLAIN && LSTAGE;
 
   // Multipliers M_q of the thread's 16 slots (round K-1 layout).  The table is
   // in tile order (kind 2: entry q n + chunk 2^13 + c for tile word c of the
