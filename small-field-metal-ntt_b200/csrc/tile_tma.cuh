@@ -653,11 +653,13 @@ struct TPass {
   // of one tile may group the warps differently with no CTA barrier between
   // them, so a warp can reach the next exchange's barrier while others still
   // wait at this one: every exchange of the pass takes its own ids (1 + the
-  // groups of the exchanges before it; ids 14 and 15 are the independent
-  // halves' pre-store barriers).
+  // groups of the exchanges between lower rounds; ids 14 and 15 are the
+  // independent halves' pre-store barriers).  They follow from the pair of
+  // rounds, not from the direction: kernels that run the inverse and then the
+  // forward layers of a tile meet the same threads at an id in both.
   __host__ __device__ static constexpr int xbase(int i) {
     int b = 1;
-    for (int j = 1; j < i; ++j) b += DESC ? xgroups(K - j, K - 1 - j) : xgroups(j - 1, j);
+    for (int j = 0; j < (DESC ? K - 1 - i : i - 1); ++j) b += xgroups(j, j + 1);
     return b;
   }
   template <int kp, int k, int BASE>
@@ -1077,7 +1079,8 @@ static_assert(TPass<BabyBear, false, Kind::C, 14>::xgroups(0, 1) == 0 && TPass<B
               "C14 exchanges: warp, 4 groups, 4 groups");
 // 13-layer passes: two grouped exchanges in a row (4 groups each), on disjoint ids
 static_assert(TPass<BabyBear, false, Kind::C, 13>::xgroups(1, 2) == 4 && TPass<BabyBear, false, Kind::C, 13>::xgroups(2, 3) == 4 &&
-                  TPass<BabyBear, false, Kind::C, 13>::xbase(3) == 5 && TPass<BabyBear, true, Kind::C, 13>::xbase(2) == 5,
+                  TPass<BabyBear, false, Kind::C, 13>::xbase(3) == 5 && TPass<BabyBear, true, Kind::C, 13>::xbase(1) == 5 &&
+                  TPass<BabyBear, true, Kind::C, 13>::xbase(2) == 1,
               "C13 exchange barrier ids");
 
 // BabyBear LSTAGE passes stage 64 KiB of twiddles besides the two tiles (one
