@@ -1469,8 +1469,15 @@ struct TExpandCols {
       if ((tid & 31u) == 0) tma::mbar_arrive(rd);
     };
     const auto all_read = [&] {
-      ok &= tma::mbar_wait(rd, phase & 1u, kWaitNs);
+      ok = tma::mbar_wait(rd, phase & 1u, kWaitNs);
       ++phase;
+    };
+    // The exchange's barrier: a thread whose wait ran out has written nothing, so
+    // what others still read stays whole, and the CTA agrees here to end.
+    const auto given_up = [&] {
+      if (!__syncthreads_or(!ok)) return false;
+      if (!ok) atomicExch(a.err, 1);
+      return true;
     };
     __syncthreads();
     has_read();
@@ -1503,11 +1510,13 @@ struct TExpandCols {
       const uint2* mt = a.mul + (chunk << kTileBits) + ct1;
       Inv::template round2<0>(xa, xb, a, tws_inv, gi, tid);
       all_read();
-      Inv::template st<0>(bufa, xa, tid);
-      Inv::template st<0>(bufb, xb, tid);
+      if (ok) {
+        Inv::template st<0>(bufa, xa, tid);
+        Inv::template st<0>(bufb, xb, tid);
+      }
       uint2 w[E];
       X1::load_mul(w, mt);
-      __syncthreads();
+      if (given_up()) return;
       Inv::template ld<1>(bufa, xa, tid);
       Inv::template ld<1>(bufb, xb, tid);
       has_read();
@@ -1528,15 +1537,17 @@ struct TExpandCols {
         }
         Fwd::template round2<1>(va, vb, af, tws_fwd, gi, tid);
         all_read();
-        Fwd::template st<1>(bufa, va, tid);
-        Fwd::template st<1>(bufb, vb, tid);
+        if (ok) {
+          Fwd::template st<1>(bufa, va, tid);
+          Fwd::template st<1>(bufb, vb, tid);
+        }
         if (q + 1 < nq) {
           X1::load_mul(w, mt + (uint64_t)(q + 1) * n);
         } else if (!last) {
           load(xa, pa, off, step);
           load(xb, two ? pa + col_bytes : pa, off, step);
         }
-        __syncthreads();
+        if (given_up()) return;
         Fwd::template ld<0>(bufa, va, tid);
         Fwd::template ld<0>(bufb, vb, tid);
         has_read();
@@ -1545,7 +1556,6 @@ struct TExpandCols {
         if (two_now) store(vb, oa + col_bytes, off, step);
       }
     }
-    if (!ok) atomicExch(a.err, 1);
   }
 };
 

@@ -259,6 +259,17 @@ __device__ __forceinline__ void producer(const CUtensorMap* min, uint32_t* ring,
   tma::wait_all();
 }
 
+// A compute warp's wait for a phase of `bar`.  false: it ran out for a lane; the
+// flag is set and the warp leaves without arriving again, so nothing of that
+// block or of later ones is stored, and the mover's next wait for the warps is
+// its last: at most one wait per thread runs out.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* err) {
+  const bool ok = tma::mbar_wait(bar, parity, kWaitNs);
+  if (__all_sync(0xffffffffu, ok)) return true;
+  atomicExch(err, 1);
+  return false;
+}
+
 // A compute warp's arrival: its words of the block are written.
 __device__ __forceinline__ void arrive_done(uint64_t* bar, uint32_t lane) {
   tma::fence_proxy_async();
@@ -304,10 +315,7 @@ struct WPass {
     for (uint32_t t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
       if (t + gridDim.x >= a.ntiles) pdl_trigger();  // the CTA's last tile
       uint32_t* buf = ring + slot * kTileWords;
-      // A wait that ran out is flagged; the words read then are whatever the
-      // buffer holds, and the warp keeps its arrivals.
-      if (!tma::mbar_wait(&bars->full[slot], use & 1u, kWaitNs)) atomicExch(a.err, 1);
-      __syncwarp();
+      if (!wt::warp_wait(&bars->full[slot], use & 1u, a.err)) return;
       uint32_t v[32];
       wt::ld_io(buf, v, l);
       wt::round<F, DESC, RA>(v, tab, l.g);
@@ -372,8 +380,7 @@ struct WExpandM31 {
     uint32_t it = 0;
     for (uint32_t t = blockIdx.x; t < a.ntiles; t += gridDim.x, ++it) {
       if (t + gridDim.x >= a.ntiles) pdl_trigger();  // the CTA's last tile
-      if (!tma::mbar_wait(&bars->full[slot], (it / wt::kRing) & 1u, kWaitNs)) atomicExch(a.err, 1);
-      __syncwarp();
+      if (!wt::warp_wait(&bars->full[slot], (it / wt::kRing) & 1u, a.err)) return;
       uint32_t x[32];
       uint32_t* buf = ring + slot * kTileWords;
       wt::ld_io(buf, x, l);
@@ -385,8 +392,7 @@ struct WExpandM31 {
       for (uint32_t q = 0; q < nq; ++q) {
         buf = ring + slot * kTileWords;
         // the buffer's previous block has left (block 0 sits where its tile arrived)
-        if (q > 0 && use > 0 && !tma::mbar_wait(&bars->empty[slot], (use - 1u) & 1u, kWaitNs)) atomicExch(a.err, 1);
-        __syncwarp();
+        if (q > 0 && use > 0 && !wt::warp_wait(&bars->empty[slot], (use - 1u) & 1u, a.err)) return;
         uint32_t v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = x[i];
