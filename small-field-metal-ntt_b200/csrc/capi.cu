@@ -642,6 +642,7 @@ int sfntt_layout(sfntt_ctx* ctx, const uint32_t* in, size_t len, uint32_t log_n,
       SFNTT_CU(cudaEventRecord(ctx->ev_stop, ctx->stream));
       SFNTT_CU(cudaMemcpyAsync(out, dout, bytes, cudaMemcpyDeviceToHost, ctx->stream));
       SFNTT_CU(cudaStreamSynchronize(ctx->stream));
+      SFNTT_TRY(device_flag(ctx));
       return elapsed_ns(ctx, ns);
     }();
   }
