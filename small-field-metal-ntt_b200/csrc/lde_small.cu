@@ -233,6 +233,13 @@ bool lde_small_fits(const sfntt_ctx* ctx, const uint32_t* in, const uint32_t* ou
                     uint32_t batch, uint32_t added_bits) {
   if (ctx->no_tma || log_n < 5 || log_n > 14 || added_bits > 4) return false;
   if (!aligned16(in) || !aligned16(out) || (in_stride & 3u) != 0) return false;
+  // Nothing orders one CTA's reads against another's stores: an input that lies
+  // in the output must be read and overwritten by the same CTA, column by column
+  // (the natural-order route, or one column); the passes take any other overlap.
+  const uintptr_t ib = reinterpret_cast<uintptr_t>(in), ob = reinterpret_cast<uintptr_t>(out);
+  const uint64_t n = 1ull << log_n, n_ext = n << added_bits;
+  const uint64_t in_bytes = 4 * ((batch - 1ull) * in_stride + n), out_bytes = 4 * batch * n_ext;
+  if (ib < ob + out_bytes && ob < ib + in_bytes && !(ib == ob && (batch == 1 || in_stride == n_ext))) return false;
   return log_n < 14 || (in != out && ((uint64_t)batch << added_bits) <= (uint64_t)ctx->sm_count);
 }
 
