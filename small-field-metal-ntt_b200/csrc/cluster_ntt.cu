@@ -1,15 +1,16 @@
 // cluster_ntt.cu -- one-launch NTT of columns of 2^13 .. 2^16 points on a
 // thread-block cluster.
 //
-// A column of n = 2^(12+X) points is split over 2^X CTAs of one cluster (16 at
-// 2^16 points: the non-portable size), CTA r owning the contiguous positions
-// [r 2^12, (r+1) 2^12) in shared memory.  Layers [0, 12) pair positions inside a
-// block and run on the tile engine's rounds (TPass<F, DESC, Kind::C, 12> on
-// 2^12-word tiles, 256 threads: registers, shared-memory exchanges).  The X cross
-// layers [12, 12+X) pair positions 2^12 apart: the points {base + k 2^12 : k <
-// 2^X} (base < 2^12) form one group, one point per block, and each thread owns
-// 16 / 2^X whole groups, so these layers run in registers.  The exchange
-// between the two parts goes through distributed shared memory.
+// A column of n = 2^(12+X) points is split over the CTAs of one cluster, CTA r
+// owning the contiguous positions [r 2^B, (r+1) 2^B) in shared memory (B = 12: 2
+// to 16 CTAs of 256 threads, 16 being the non-portable size; B = 13: 1 to 8 of
+// 512).  Layers [0, 12) pair positions inside a block and run on the tile
+// engine's rounds (TPass<F, DESC, Kind::C, 12>: registers, shared-memory
+// exchanges).  The X cross layers [12, 12+X) pair positions 2^12 apart: the
+// points {base + k 2^12 : k < 2^X} (base < 2^12) form one group, one or two
+// points per block, and each thread owns 16 / 2^X whole groups, so these layers
+// run in registers.  The exchange between the two parts goes through distributed
+// shared memory.
 //
 //   inverse (layers ascending): load the block, in-block layers, cluster
 //     barrier, gather the groups from the cluster's blocks, cross layers and
@@ -31,6 +32,8 @@
 // one column from a graph, 2^13-word blocks with the twiddles fetched layer by
 // layer -> now: BabyBear 2^13 6.7 / 7.1 -> 4.0 / 4.5 us, 2^16 7.9 / 8.4 -> 5.0 /
 // 5.3 us; M31 2^13 6.1 / 6.0 -> 4.1 / 4.4 us, 2^16 7.2 / 7.4 -> 5.4 / 5.3 us.
+// Batches that fill the SMs take the wider blocks in places, launched plainly
+// and with the cross twiddles read layer by layer (see cluster_form).
 #include <cooperative_groups.h>
 
 #include "context.hpp"
@@ -42,16 +45,19 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-template <class F, bool DESC, int X>
+// B: log2 of a block's words, 12 or 13.
+template <class F, bool DESC, int X, int B>
 struct ClusterNtt {
-  using TP = TPass<F, DESC, Kind::C, 12, false, false, false, false, 12>;
-  static constexpr int CS = 1 << X;        // CTAs per column
-  static constexpr int G = 1 << X;         // points per cross group, one per block
-  static constexpr int GPT = 16 / G;       // groups per thread
+  static_assert(B == 12 || B == 13, "blocks of 2^12 or 2^13 words");
+  using TP = TPass<F, DESC, Kind::C, 12, false, false, false, false, B == 12 ? 12 : 0>;
+  static constexpr int PPB = 1 << (B - 12);  // points of a cross group per block
+  static constexpr int CS = (1 << X) / PPB;  // CTAs per column
+  static constexpr int G = 1 << X;           // points per cross group
+  static constexpr int GPT = 16 / G;         // groups per thread
   static constexpr uint32_t NT = TP::NT;
   static constexpr uint32_t LOG_N = 12 + X;
   static constexpr uint32_t BASES = 4096u / CS;  // group bases per CTA
-  static_assert(NT == 256 && TP::E == 16 && BASES == GPT * NT && TP::TWORDS == 4096u,
+  static_assert(NT == (B == 12 ? 256 : 512) && TP::E == 16 && BASES == GPT * NT && TP::TWORDS == 1u << B,
                 "one thread: 16 points in whole groups");
 
   // Butterflies of one group and layer j, low points in order: cross_at(k, j)
@@ -72,13 +78,13 @@ struct ClusterNtt {
     asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
     return r;
   }
-  __device__ static __forceinline__ uint2 cross_tw(const uint2* tw, uint32_t base, int k, int j) {
+  __device__ static __forceinline__ const uint2* cross_at_mem(const uint2* tw, uint32_t base, int k, int j) {
     const uint32_t L = 12u + (uint32_t)j;
     if constexpr (F::kMontgomery) {
-      return ld_tw(tw + ((1u << L) - 1u) + base + ((uint32_t)(k & ((1 << j) - 1)) << 12));
+      return tw + ((1u << L) - 1u) + base + ((uint32_t)(k & ((1 << j) - 1)) << 12);
     } else {
       const uint32_t n = 1u << LOG_N;
-      return ld_tw(tw + (n - (n >> L)) + ((uint32_t)k >> (j + 1)));
+      return tw + (n - (n >> L)) + ((uint32_t)k >> (j + 1));
     }
   }
 
@@ -92,14 +98,14 @@ struct ClusterNtt {
         for (int k = 0; k < G; ++k) {
           if (k & (1 << j)) continue;
           const int first = F::kMontgomery ? (k & ((1 << j) - 1)) : ((k >> (j + 1)) << (j + 1));
-          if (k == first) t[gi * CT + cross_at(k, j)] = cross_tw(tw, base0 + (uint32_t)gi * NT, k, j);
+          if (k == first) t[gi * CT + cross_at(k, j)] = ld_tw(cross_at_mem(tw, base0 + (uint32_t)gi * NT, k, j));
         }
   }
 
   // The X cross layers on the thread's groups (forward: descending, inverse:
-  // ascending, then n^-1); canonical values out.
-  __device__ static __forceinline__ void cross(uint32_t (&v)[16], const uint2 (&t)[CN], uint32_t scale_w,
-                                               uint32_t scale_ws) {
+  // ascending, then n^-1); canonical values out.  B = 13: twiddles from memory.
+  __device__ static __forceinline__ void cross(uint32_t (&v)[16], const uint2 (&t)[CN], uint32_t base0, const uint2* tw,
+                                               uint32_t scale_w, uint32_t scale_ws) {
 #pragma unroll
     for (int gi = 0; gi < GPT; ++gi) {
 #pragma unroll
@@ -108,8 +114,10 @@ struct ClusterNtt {
 #pragma unroll
         for (int k = 0; k < G; ++k) {
           if (k & (1 << j)) continue;
-          butterfly<F, DESC>(v[gi * G + k], v[gi * G + (k | (1 << j))],
-                             t[(F::kMontgomery ? gi * CT : 0) + cross_at(k, j)]);
+          uint2 w;
+          if constexpr (B == 12) w = t[(F::kMontgomery ? gi * CT : 0) + cross_at(k, j)];
+          else w = __ldg(cross_at_mem(tw, base0 + (uint32_t)gi * NT, k, j));
+          butterfly<F, DESC>(v[gi * G + k], v[gi * G + (k | (1 << j))], w);
         }
       }
     }
@@ -134,9 +142,10 @@ struct ClusterNtt {
     a.log_n = LOG_N;
     a.lo = 0;
     a.batch = 1;
-    a.log_tpc = (uint32_t)(X - 1);
+    a.log_tpc = (uint32_t)(LOG_N - B);
+    if constexpr (TP::kRound0Copy) a.tw0 = tw + n;  // M31 tables with n >= 2^13 carry it
     TileCoord g{};
-    g.pos_base = rank << 12;
+    g.pos_base = rank << B;
     const uint32_t base0 = rank * BASES + tid;  // group gi: base0 + gi NT
     uint2 ctw[CN];
     // The tables do not depend on the previous kernel: under programmatic
@@ -144,7 +153,7 @@ struct ClusterNtt {
     pdl_trigger();
     if constexpr (TP::kStaged) {
       TP::stage_twiddles(tws, tw, tid);
-    } else {
+    } else if constexpr (B == 12) {
       // layers 0..7 of the block are 255 lines of 128 bytes, one per thread;
       // the last thread takes layer 8's 64 bytes and what follows them
       const uint32_t L = tid < 255u ? 7u - (31u - __clz(255u - tid)) : 8u;
@@ -156,7 +165,7 @@ struct ClusterNtt {
         asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(word) : "l"(p + i));
       }
     }
-    load_cross(ctw, base0, tw);
+    if constexpr (B == 12) load_cross(ctw, base0, tw);
     pdl_wait();
     uint32_t v[16];
     if constexpr (DESC) {
@@ -168,14 +177,14 @@ struct ClusterNtt {
       for (int gi = 0; gi < GPT; ++gi)
 #pragma unroll
         for (int k = 0; k < G; ++k) v[gi * G + k] = col[base0 + (uint32_t)gi * NT + ((uint32_t)k << 12)];
-      cross(v, ctw, 0u, 0u);
+      cross(v, ctw, base0, tw, 0u, 0u);
       asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 #pragma unroll
       for (int gi = 0; gi < GPT; ++gi)
 #pragma unroll
         for (int k = 0; k < G; ++k) {
-          uint32_t* owner = cluster.map_shared_rank(tile, (unsigned)k);
-          owner[TP::sw(base0 + (uint32_t)gi * NT)] = v[gi * G + k];
+          uint32_t* owner = cluster.map_shared_rank(tile, (unsigned)(k / PPB));
+          owner[TP::sw(base0 + (uint32_t)gi * NT + ((uint32_t)(k % PPB) << 12))] = v[gi * G + k];
         }
       cluster.sync();  // every block complete (and the staged twiddles visible)
       TP::template ld<TP::kFirst>(tile, v, tid);
@@ -206,14 +215,14 @@ struct ClusterNtt {
       for (int gi = 0; gi < GPT; ++gi)
 #pragma unroll
         for (int k = 0; k < G; ++k) {
-          const uint32_t* owner = cluster.map_shared_rank(tile, (unsigned)k);
-          v[gi * G + k] = owner[TP::sw(base0 + (uint32_t)gi * NT)];
+          const uint32_t* owner = cluster.map_shared_rank(tile, (unsigned)(k / PPB));
+          v[gi * G + k] = owner[TP::sw(base0 + (uint32_t)gi * NT + ((uint32_t)(k % PPB) << 12))];
         }
       // No block may leave while another still reads it: arrive once the
       // reads are performed (release), wait only before leaving, so the
       // barrier overlaps the cross layers and the stores.
       asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-      cross(v, ctw, scale_w, scale_ws);
+      cross(v, ctw, base0, tw, scale_w, scale_ws);
 #pragma unroll
       for (int gi = 0; gi < GPT; ++gi)
 #pragma unroll
@@ -223,18 +232,18 @@ struct ClusterNtt {
   }
 };
 
-template <class F, bool DESC, int X>
-__global__ void __launch_bounds__(ClusterNtt<F, DESC, X>::NT, 3)
+template <class F, bool DESC, int X, int B>
+__global__ void __launch_bounds__(ClusterNtt<F, DESC, X, B>::NT, B == 12 ? 3 : 1)
 cluster_ntt_kernel(uint32_t* d, const uint2* tw, uint32_t scale_w, uint32_t scale_ws) {
-  ClusterNtt<F, DESC, X>::run(d, tw, scale_w, scale_ws);
+  ClusterNtt<F, DESC, X, B>::run(d, tw, scale_w, scale_ws);
 }
 
-template <class F, bool DESC, int X>
-Status launch_cluster(sfntt_ctx* ctx, uint32_t* d, uint32_t batch, const uint2* tw, uint32_t scale_w,
+template <class F, bool DESC, int X, int B>
+Status launch_cluster(sfntt_ctx* ctx, uint32_t* d, uint32_t batch, const uint2* tw, uint32_t scale_w, bool early,
                       cudaStream_t s) {
-  using C = ClusterNtt<F, DESC, X>;
+  using C = ClusterNtt<F, DESC, X, B>;
   constexpr int smem = 4 * (int)C::TP::TWORDS + 8 * (int)C::TP::TW_ENTRIES + 1024;
-  auto kern = cluster_ntt_kernel<F, DESC, X>;
+  auto kern = cluster_ntt_kernel<F, DESC, X, B>;
   static std::atomic<uint64_t> smem_done{0};
   if (C::CS > 8 && !(smem_done.load(std::memory_order_acquire) & (1ull << (ctx->device & 63))))
     SFNTT_CU(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -255,43 +264,128 @@ Status launch_cluster(sfntt_ctx* ctx, uint32_t* d, uint32_t batch, const uint2* 
 #ifdef SFNTT_NO_PDL
   cfg.numAttrs = 1;
 #else
-  cfg.numAttrs = 2;
+  cfg.numAttrs = early ? 2 : 1;
 #endif
   const uint32_t scale_ws = (uint32_t)(((uint64_t)scale_w << 32) / F::P);
   launch_begin(ctx, s);
   SFNTT_CU(cudaLaunchKernelEx(&cfg, kern, d, tw, scale_w, scale_ws));
   static const std::string name = std::string(F::kTag) + (DESC ? "_fwd" : "_inv") + "_cluster" +
-                                  std::to_string(C::CS);
+                                  std::to_string(C::CS) + (B == 13 ? "w" : "");
   return launch_check(ctx, name.c_str(), s, ((uint64_t)batch << C::LOG_N) * 8u);
+}
+
+// Clusters of 2^13-word blocks that run at once with one CTA per SM.
+template <class F, bool DESC, int X>
+uint32_t wide_clusters(const sfntt_ctx* ctx) {
+  using C = ClusterNtt<F, DESC, X, 13>;
+  static std::atomic<int> known[64];  // per device: clusters + 1
+  std::atomic<int>& k = known[ctx->device & 63];
+  if (const int n = k.load(std::memory_order_relaxed)) return (uint32_t)(n - 1);
+  auto kern = cluster_ntt_kernel<F, DESC, X, 13>;
+  constexpr int more_than_half = 116 << 10;  // of an SM's shared memory
+  static std::atomic<uint64_t> smem_done{0};
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)C::CS);
+  cfg.blockDim = dim3(C::NT);
+  cfg.dynamicSmemBytes = more_than_half;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)C::CS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (!smem_limit_once(kern, more_than_half, ctx->device, smem_done).ok() ||
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  k.store(n + 1, std::memory_order_relaxed);
+  return (uint32_t)n;
+}
+
+// Block size and launch of a batch, by blocks of 2^12 words per SM (us per call
+// in a graph of calls: 2^12-word blocks launched early, plainly, 2^13-word blocks).
+//   BabyBear / KoalaBear: up to 0.76, 2^12 early (2^14 x 18 4.2, 6.9, 7.2; 2^16 x 4
+// 4.7, 7.4, 8.1).  Above, CTAs launched early pack onto the SMs that come free
+// first, and without that two of them on an SM lose to one of 2^13 words as long
+// as each of those has an SM (2^14 x 41 8.5, 8.5, 7.3; 2^15 x 27 9.3, 9.1, 8.0; 2^16
+// x 15 10.0, 10.9, 8.3), but for the inverse of 2^16 points (x 10 6.9, 9.9, 9.0; x 15
+// 9.1, 11.8, 9.1).  Then 2^12 early again (2^15 x 36 9.7, 10.3, 10.9; inverse 9.3,
+// 11.6, 15.6).  2^13 points: only batches that 2^12 early suits come here.
+//   M31, whose twiddles come through L1: early up to 0.35 (2^16 x 3 5.0, 5.2, 7.3),
+// plainly up to 1.4 (2^14 x 24 7.7, 4.8, 6.7; 2^16 x 12 9.3, 7.5, 7.5), wide while
+// each has an SM (2^14 x 74 8.5, 8.6, 6.9), then early (2^15 x 37 9.0, 8.8, 13);
+// pairs that divide evenly early (2^13 x 148 6.0, 6.4, 6.7).
+// On several streams the forms differ by a tenth (8 streams, 2^14 x 55 4.0, 4.0,
+// 3.7), but for M31 around 1.4 (2^16 x 12 4.1 against 5.4 with wide blocks).
+struct ClusterForm { bool wide, early; };
+template <class F, bool DESC, int X>
+constexpr bool kMayBeWide = !F::kMontgomery || (X > 1 && (X < 4 || DESC));
+template <class F, bool DESC, int X>
+ClusterForm cluster_form(const sfntt_ctx* ctx, uint32_t batch) {
+  const uint64_t sms = (uint64_t)ctx->sm_count, blocks = (uint64_t)batch << X;
+  if constexpr (!kMayBeWide<F, DESC, X>) {
+    return {false, true};
+  } else {
+    const bool wide = blocks <= 2 * sms && batch <= wide_clusters<F, DESC, X>(ctx);
+    if (F::kMontgomery) return {wide && 25 * blocks > 19 * sms, !wide || 25 * blocks <= 19 * sms};
+    if (X == 1 && blocks % sms == 0) return {false, true};
+    if (5 * blocks <= 7 * sms) return {false, 20 * blocks <= 7 * sms};
+    return {wide, !wide};
+  }
+}
+
+template <class F, bool DESC, int X>
+Status launch_blocks(sfntt_ctx* ctx, uint32_t* d, uint32_t batch, const uint2* tw, uint32_t scale_w, cudaStream_t s) {
+  const ClusterForm f = cluster_form<F, DESC, X>(ctx, batch);
+  if constexpr (kMayBeWide<F, DESC, X>) {
+    if (f.wide) return launch_cluster<F, DESC, X, 13>(ctx, d, batch, tw, scale_w, f.early, s);
+  }
+  return launch_cluster<F, DESC, X, 12>(ctx, d, batch, tw, scale_w, f.early, s);
 }
 
 template <class F, bool DESC>
 Status cluster_dispatch(sfntt_ctx* ctx, uint32_t* d, uint32_t log_n, uint32_t batch, const uint2* tw,
                         uint32_t scale_w, cudaStream_t s) {
   switch (log_n) {
-    case 13: return launch_cluster<F, DESC, 1>(ctx, d, batch, tw, scale_w, s);
-    case 14: return launch_cluster<F, DESC, 2>(ctx, d, batch, tw, scale_w, s);
-    case 15: return launch_cluster<F, DESC, 3>(ctx, d, batch, tw, scale_w, s);
-    case 16: return launch_cluster<F, DESC, 4>(ctx, d, batch, tw, scale_w, s);
+    case 13: return launch_blocks<F, DESC, 1>(ctx, d, batch, tw, scale_w, s);
+    case 14: return launch_blocks<F, DESC, 2>(ctx, d, batch, tw, scale_w, s);
+    case 15: return launch_blocks<F, DESC, 3>(ctx, d, batch, tw, scale_w, s);
+    case 16: return launch_blocks<F, DESC, 4>(ctx, d, batch, tw, scale_w, s);
     default: return {SFNTT_INVALID_ARGUMENT, "cluster NTT: 2^13 .. 2^16 points"};
   }
 }
 
 }  // namespace
 
-// Against the passes (forward + inverse): BabyBear / KoalaBear win while the
-// blocks fit one wave of three per SM (2^15 x 40 20 against 27 us, 2^14 x 80 19
-// against 22 us; 2^14 x 140 27 against 22 us).  M31's passes over shorter columns
-// read their twiddles from L2 or stage them per tile, so it wins there for far
-// longer (2^14 x 600 75 against 89 us, 2^13 x 1000 59 against 71 us, 2^15 x 290 79
-// against 81 us).  2^16 points keep the line of the 2^13-word blocks, two tiles
-// per SM (x 9 16 against 20 us, x 24 26 against 28 us, M31 26 against 32 us; at the
-// very end, x 37, 36 against 29 us and M31 35 against 32 us).
+// Against the passes (forward + inverse, us, passes and clusters).  BabyBear /
+// KoalaBear: 2^13 points are one pass, so the clusters take what they start early
+// without packing, up to 5/8 blocks of 2^12 words per SM and whole waves of up to
+// three (x 46 10.3, 9.3; x 74 10.5, 8.8; x 120 10.9, 15.1); longer columns up to
+// three per SM (2^14 x 41 18.3, 15.4; x 100 20.2, 19.0; 2^15 x 50 25.2, 23.1; 2^16 x
+// 24 25.5, 24.8; x 31 26.1, 26.9).
+//   M31's passes read their twiddles from L2 or stage them per tile, so it wins
+// longer.  A pass takes two tiles of 2^13 words per SM and round, a round filled or
+// not, the clusters a time that grows with the batch: up to where each of the
+// first rounds is about three quarters full, in the fourth where it has just begun
+// (2^14 x 148 23.7, 28.8; x 172 37.2, 30.3; x 296 37.8, 46.0; 2^15 x 111 46.0, 41.3;
+// x 222 58.5, 71.9; 2^13 x 592 35.1, 39.9; x 641 48.6, 43.3).  2^16 points three
+// blocks per SM, as the others (x 24 28.8, 25.4; x 33 29.2, 31.0).
+//   The last batch of each range, whole waves, stays on the clusters, where it has
+// been since they were built (2^16 x 37 BabyBear 26.2, 34.8; M31 2^14 x 592 65.9, 83.6).
 bool cluster_ntt_fits(const sfntt_ctx* ctx, int field, uint32_t log_n, uint32_t batch, const void* d) {
   if (ctx->no_cluster || log_n < 13 || log_n > 16 || batch == 0) return false;
   if ((reinterpret_cast<uintptr_t>(d) & 15u) != 0) return false;
-  const uint64_t waves = log_n == 16 ? 4 : is_monty(field) ? 3 : 16;
-  return ((uint64_t)batch << (log_n - 12)) <= waves * (uint64_t)ctx->sm_count;
+  const uint64_t blocks = (uint64_t)batch << (log_n - 12), sms = (uint64_t)ctx->sm_count;
+  const uint64_t last = (log_n == 16 ? 4 : is_monty(field) ? 3 : 16) * sms;
+  if (blocks >= last) return blocks == last;
+  if (log_n == 16) return blocks <= 3 * sms;
+  if (is_monty(field)) return log_n > 13 || 8 * blocks <= 5 * sms || blocks % sms == 0;
+  const uint64_t rounds = (blocks + 4 * sms - 1) / (4 * sms);
+  const uint64_t tenths = rounds == 4 ? 31 : log_n == 14 ? 30 : log_n == 15 ? 34 : 33;  // blocks per SM and round
+  return 10 * blocks <= tenths * rounds * sms;
 }
 
 Status cluster_ntt_dev(sfntt_ctx* ctx, int field, bool inverse, uint32_t* d, uint32_t log_n, uint32_t batch,
