@@ -357,6 +357,25 @@ Status bitrev_cols_dev(sfntt_ctx* ctx, const uint32_t* in, uint64_t in_stride, u
   return launch_check(ctx, "layout_bitrev_pairs", s, total * 8);
 }
 
+// From how many words on bit-reversed rows of `batch` columns take the TMA tiles
+// (us, register tiles and TMA tiles).  A row is a copy of its own, or words where
+// it is no multiple of 16 bytes, so few columns never pay (2^20 x 64 137, 164).
+// 65 to 72 and 129 to 144 columns leave four CTAs per SM, 73 to 96 and 145 to 192
+// three, the others two, whose copies take longer to hide; and one column past
+// 128 the register tiles are half empty.  2^16 x 72 10.7, 9.3, x 96 11.3, 11.5, x
+// 128 11.1, 16.1, x 129 17.7, 14.1, x 250 28.2, 29.8, x 256 27.7, 24.3; 2^15 x 128
+// 6.1, 8.9, x 129 9.7, 8.9, x 192 9.9, 8.6, x 250 11.4, 15.8; 2^17 x 73 21.4, 20.2, x
+// 99 29.4, 34.1, x 128 27.8, 30.5; 2^18 x 99 63.7, 67.1, x 100 61.7, 55.2, x 127 72.7,
+// 67.9; 2^19 x 99 143, 129.
+uint64_t bitrev_rows_from(uint32_t batch) {
+  const bool copies = (batch & 3u) == 0;
+  if (batch < 72) return ~0ull;
+  if (batch == 72 || (batch > 128 && batch <= 192)) return 1ull << 22;
+  if (batch <= 96) return 1ull << 23;
+  if (batch <= 128) return copies ? 3ull << 23 : 1ull << 25;
+  return copies ? 3ull << 22 : 1ull << 24;
+}
+
 Status layout_dev(sfntt_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t log_n, uint32_t batch, int flags,
                   cudaStream_t s) {
   if (flags & ~(SFNTT_LAYOUT_NATURAL | SFNTT_LAYOUT_ROW_MAJOR)) return {SFNTT_INVALID_ARGUMENT, "unknown layout flags"};
@@ -380,10 +399,9 @@ Status layout_dev(sfntt_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t lo
   // The TMA tiles pay from 2^22 words on (below, the launch and the first
   // tile's latency are the cost: 2^15 x 128 9.3 us here, 10.0 us there).  Above
   // 256 columns a tile no longer holds whole rows (2^19 x 301 in column blocks:
-  // 333 us against 283 us), and bit-reversed rows of few columns are many small
-  // copies (2^20 x 64: 164 us against 137 us; 2^18 x 75: 42 us against 48 us).
-  if (total >= (1ull << 22) && batch <= kRowsMaxLines && (!natural || batch >= 72) && log_n >= 5 && aligned16(in) &&
-      aligned16(out)) {
+  // 333 us against 283 us).
+  if (total >= (natural ? bitrev_rows_from(batch) : 1ull << 22) && batch <= kRowsMaxLines && log_n >= 5 &&
+      aligned16(in) && aligned16(out)) {
     RowsArgs ra{};
     while (ra.lk < log_n - 5 && (batch << (ra.lk + 1)) <= kRowsMaxLines) ++ra.lk;
     ra.out = out; ra.log_n = log_n; ra.batch = batch; ra.bitrev = natural ? 1u : 0u;
@@ -401,7 +419,7 @@ Status layout_dev(sfntt_ctx* ctx, const uint32_t* in, uint32_t* out, uint32_t lo
     const uint32_t grid = std::min<uint32_t>(ra.tiles, (uint32_t)ctx->sm_count * per_sm);
     launch_begin(ctx, s);
     transpose_tma_kernel<<<grid, kRowsThreads, smem, s>>>(map, ra);
-    return launch_check(ctx, name, s, total * 8);
+    return launch_check(ctx, natural ? "layout_transpose_bitrev_tma" : "layout_transpose_tma", s, total * 8);
   }
   launch_begin(ctx, s);
   if (log_n >= 5 && batch >= kWideCols) {
