@@ -71,6 +71,19 @@ static uint32_t inv_n_canonical(int field, uint32_t log_n) {
   return (uint32_t)x;
 }
 
+// Does a batch of short columns that leaves its last tile part empty pay on the
+// tile engine?  From 2^18 words on (tma_pass_ok), but for M31's 2^8 .. 2^11 points,
+// which read a twiddle pair from memory per butterfly there (inverse 2^11 x 147
+// 4.9 -> 5.7 us, x 239 6.1 -> 5.7 us; 2^9 x 955 4.5 -> 5.4 us, x 1783 6.7 -> 5.6
+// us), and the inverse of 2^9 points (BabyBear x 725 4.0 -> 4.2 us, x 1261 5.1 ->
+// 4.2 us).
+static bool ragged_pays(int field, bool inverse, uint32_t log_n, uint32_t batch) {
+  const uint64_t words = (uint64_t)batch << log_n;
+  if (log_n >= 12 || words % kTileWords == 0) return true;
+  if (field == SFNTT_M31 && log_n >= 8) return words >= (log_n == 9 ? 9ull << 16 : 3ull << 17);
+  return !(inverse && log_n == 9) || words >= 3ull << 17;
+}
+
 // Runs layers [a, b) of the 2^log_n-point network (forward: descending, CT/GS
 // per field; inverse: ascending) on `batch` columns.  The first pass reads
 // `in`, later passes work in place on `out`.  scale_w != 0 multiplies every
@@ -102,7 +115,7 @@ Status layers_dev(sfntt_ctx* ctx, int field, bool inverse, const uint32_t* in, u
       // M31 contiguous passes over many columns: a tile's per-block twiddles
       // (twice its own size in L2 reads) are staged once for all its columns
       r.lstage = !is_monty(field) && r.contiguous && log_n >= 13 && batch >= 16;
-      ok = tma_pass_ok(r);
+      ok = tma_pass_ok(r) && (!r.contiguous || ragged_pays(field, inverse, log_n, batch));
     }
     if (ok && is_monty(field)) {
       // Strided passes either use per-position twiddles (self-contained) or,
