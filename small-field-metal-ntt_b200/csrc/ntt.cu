@@ -362,8 +362,10 @@ namespace {
 // words, so 16 KiB per block are in flight from its first instruction on; the
 // grid covers the array once.  Montgomery conversion of 2^19 x 100 words: 68
 // us, 6.1 TB/s, against 119 us, 3.5 TB/s, with one word per thread and step
-// in a grid of 16 CTAs per SM, the form that buffers without 16-byte
-// alignment still take.
+// in a grid of 16 CTAs per SM.  Arrays of up to 2^18 words, where blocks of 16
+// KiB leave SMs idle, keep that form (2^14 words 1.3 against 1.6 us, 2^18 1.55
+// against 1.66 us; 3 2^17 2.06 against 1.69 us), and so do buffers without
+// 16-byte alignment.
 constexpr uint32_t kMapThreads = 256;
 constexpr uint32_t kMapVec = 4;
 constexpr uint32_t kMapWords = kMapThreads * kMapVec * 4;
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(kMapThreads) map_word_kernel(const uint32_t* a
                                                                uint64_t n, Fn fn) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     if constexpr (TWO) out[i] = fn(a[i], b[i]);
-    else out[i] = fn(a[i]);
+    else out[i] = fn(out[i]);  // in place: a is out
   }
 }
 
@@ -453,16 +455,17 @@ uint32_t grid_for(sfntt_ctx* ctx, uint64_t n) {
 }
 
 template <bool TWO, class Fn>
-Status map_words(sfntt_ctx* ctx, const char* name, const uint32_t* a, const uint32_t* b, uint32_t* out, uint64_t n,
-                 Fn fn, cudaStream_t s) {
+Status map_words(sfntt_ctx* ctx, const char* name, const char* vec_name, const uint32_t* a, const uint32_t* b,
+                 uint32_t* out, uint64_t n, Fn fn, cudaStream_t s) {
   if (n == 0) return {};
+  const uint64_t blocks = (n + kMapWords - 1) / kMapWords, bytes = n * (TWO ? 12u : 8u);
   launch_begin(ctx, s);
-  const uint64_t blocks = (n + kMapWords - 1) / kMapWords;
-  if (aligned16(a) && aligned16(b) && aligned16(out) && blocks < (1ull << 31))
+  if (n > (1ull << 18) && aligned16(a) && aligned16(b) && aligned16(out) && blocks < (1ull << 31)) {
     map_vec_kernel<TWO, Fn><<<(uint32_t)blocks, kMapThreads, 0, s>>>(a, b, out, n, fn);
-  else
-    map_word_kernel<TWO, Fn><<<grid_for(ctx, n), kMapThreads, 0, s>>>(a, b, out, n, fn);
-  return launch_check(ctx, name, s, n * (TWO ? 12u : 8u));
+    return launch_check(ctx, vec_name, s, bytes);
+  }
+  map_word_kernel<TWO, Fn><<<grid_for(ctx, n), kMapThreads, 0, s>>>(a, b, out, n, fn);
+  return launch_check(ctx, name, s, bytes);
 }
 
 }  // namespace
@@ -470,14 +473,14 @@ Status map_words(sfntt_ctx* ctx, const char* name, const uint32_t* a, const uint
 Status scale_dev(sfntt_ctx* ctx, int field, uint32_t* d, uint64_t n, uint32_t w, cudaStream_t s) {
   return with_field(field, [&](auto fld) -> Status {
     using F = decltype(fld);
-    return map_words<false>(ctx, "scale", d, nullptr, d, n, ScaleFn<F>{w, host::shoup(w, F::P)}, s);
+    return map_words<false>(ctx, "scale", "scale_vec", d, nullptr, d, n, ScaleFn<F>{w, host::shoup(w, F::P)}, s);
   });
 }
 
 Status pointwise_mul_dev(sfntt_ctx* ctx, int field, const uint32_t* a, const uint32_t* b, uint32_t* out, size_t n,
                          cudaStream_t s) {
   return with_field(field, [&](auto fld) -> Status {
-    return map_words<true>(ctx, "pointwise_mul", a, b, out, n, MulFn<decltype(fld)>{}, s);
+    return map_words<true>(ctx, "pointwise_mul", "pointwise_mul_vec", a, b, out, n, MulFn<decltype(fld)>{}, s);
   });
 }
 
@@ -485,8 +488,8 @@ Status monty_convert_dev(sfntt_ctx* ctx, int field, bool to, uint32_t* d, size_t
   if (!is_monty(field)) return {SFNTT_INVALID_ARGUMENT, "Montgomery conversion needs BabyBear or KoalaBear"};
   return with_monty(field, [&](auto fld) -> Status {
     using F = decltype(fld);
-    return to ? map_words<false>(ctx, "to_monty", d, nullptr, d, n, MontyFn<F, true>{}, s)
-              : map_words<false>(ctx, "from_monty", d, nullptr, d, n, MontyFn<F, false>{}, s);
+    return to ? map_words<false>(ctx, "to_monty", "to_monty_vec", d, nullptr, d, n, MontyFn<F, true>{}, s)
+              : map_words<false>(ctx, "from_monty", "from_monty_vec", d, nullptr, d, n, MontyFn<F, false>{}, s);
   });
 }
 
