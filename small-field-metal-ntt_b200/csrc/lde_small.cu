@@ -191,13 +191,26 @@ Status launch(sfntt_ctx* ctx, SmallLdeArgs a, bool split, cudaStream_t s) {
   const uint32_t per_sm = std::min<uint32_t>(L::kCtasPerSm, 233472u / (uint32_t)(L::kSmemBytes + 1024));
   const uint32_t room = per_sm * (uint32_t)ctx->sm_count;
   dim3 grid(std::min<uint32_t>(a.tiles, room));
-  // Blocks of a column on separate CTAs while every CTA still has a place
-  // (repeating the inverse costs nothing on idle SMs); not when the input lies
-  // in the output columns, which another CTA would be overwriting.
+  // Output blocks of a column on separate CTAs, each repeating the inverse, in the
+  // split that takes the fewest transforms in a row: while every CTA has a place
+  // that costs nothing, and past that it evens out a last round of few tiles (M31
+  // 2^13 x 150 16x, one CTA per SM: two rounds of 17 transforms 147 us, five of 5
+  // 110 us; 2^12 x 150 16x, two per SM: 62 -> 45 us).  Several rounds of two or more
+  // CTAs per SM fill in by themselves (2^12 x 400 4x 29.5 against 33 us split).  Not
+  // when the input lies in the output columns, which another CTA would overwrite.
   if (split) {
-    uint32_t y = 1;
-    while (y < (1u << a.log_q) && (uint64_t)a.tiles * (2 * y) <= room) y *= 2;
-    grid.y = y;
+    const uint32_t nq = 1u << a.log_q;
+    const bool uneven = per_sm == 1 || a.tiles <= room;
+    uint64_t best = 0;
+    for (uint32_t y = 1; y <= nq; y *= 2) {
+      const uint64_t rounds = ((uint64_t)a.tiles * y + room - 1) / room;
+      const uint64_t row = rounds * (1u + nq / y);
+      if (y == 1 || (rounds == 1 && row < best) || (uneven && 20 * row < 19 * best)) {
+        best = row;
+        grid.x = y == 1 ? std::min<uint32_t>(a.tiles, room) : a.tiles;
+        grid.y = y;
+      }
+    }
   }
   launch_begin(ctx, s);
   SFNTT_CU(launch_pdl(kern, grid, L::NT, L::kSmemBytes, s, (uint64_t)grid.x * grid.y <= 16, a));
