@@ -371,8 +371,8 @@ Status cluster_dispatch(sfntt_ctx* ctx, uint32_t* d, uint32_t log_n, uint32_t ba
 // not, the clusters a time that grows with the batch: up to where each of the
 // first rounds is about three quarters full, in the fourth where it has just begun
 // (2^14 x 148 23.7, 28.8; x 172 37.2, 30.3; x 296 37.8, 46.0; 2^15 x 111 46.0, 41.3;
-// x 222 58.5, 71.9; 2^13 x 592 35.1, 39.9; x 641 48.6, 43.3).  2^16 points three
-// blocks per SM, as the others (x 24 28.8, 25.4; x 33 29.2, 31.0).
+// x 222 58.5, 71.9; 2^13 x 592 35.1, 39.9; x 641 48.6, 43.3).  2^16 points 3.1
+// blocks per SM (x 24 28.8, 25.4; x 28 29.1, 27.0; x 33 29.2, 31.0).
 //   The last batch of each range, whole waves, stays on the clusters, where it has
 // been since they were built (2^16 x 37 BabyBear 26.2, 34.8; M31 2^14 x 592 65.9, 83.6).
 bool cluster_ntt_fits(const sfntt_ctx* ctx, int field, uint32_t log_n, uint32_t batch, const void* d) {
@@ -381,7 +381,7 @@ bool cluster_ntt_fits(const sfntt_ctx* ctx, int field, uint32_t log_n, uint32_t 
   const uint64_t blocks = (uint64_t)batch << (log_n - 12), sms = (uint64_t)ctx->sm_count;
   const uint64_t last = (log_n == 16 ? 4 : is_monty(field) ? 3 : 16) * sms;
   if (blocks >= last) return blocks == last;
-  if (log_n == 16) return blocks <= 3 * sms;
+  if (log_n == 16) return 10 * blocks <= 31 * sms;
   if (is_monty(field)) return log_n > 13 || 8 * blocks <= 5 * sms || blocks % sms == 0;
   const uint64_t rounds = (blocks + 4 * sms - 1) / (4 * sms);
   const uint64_t tenths = rounds == 4 ? 31 : log_n == 14 ? 30 : log_n == 15 ? 34 : 33;  // blocks per SM and round

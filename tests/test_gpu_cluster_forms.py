@@ -18,7 +18,7 @@ NTT = {"bb": (sfntt.BbCudaCtGsR4, O.BB_P, O.bb_forward, O.bb_inverse),
 # per size: batches next to 0.35, 0.76, 1, 1.4 and 2 blocks of 2^12 words per SM (148
 # SMs), and to the clusters of wide blocks that run at once
 BATCHES = {13: [25, 26, 46, 47, 74, 75, 103, 104, 148, 149], 14: [12, 13, 28, 29, 51, 52, 71, 74, 75, 112, 300],
-           15: [6, 7, 14, 15, 25, 26, 33, 34], 16: [3, 4, 7, 8, 12, 13, 15, 16, 27, 28]}
+           15: [6, 7, 14, 15, 25, 26, 33, 34], 16: [3, 4, 7, 8, 12, 13, 15, 16, 28, 29]}
 CASES = [(f, log_n, b) for f in sorted(NTT) for log_n, bs in BATCHES.items() for b in bs]
 
 
