@@ -1423,8 +1423,9 @@ struct TExpand {
 // input.  A warp waits before it writes an exchange until all have read the one
 // before (an mbarrier that each warp arrives on after its reads, so the wait is
 // over by the time a round's layers are done: 2 % of an LDE against a CTA barrier).
-// A row prefetched into L2 a tile ahead changed nothing.  Integer-multiply pipe
-// 62 % busy, 10.2 warp instructions per warp-butterfly (one column: 63 %, 10.5).
+// A row prefetched into L2 a tile ahead changed nothing.  2^20 x 16, 8x: integer-
+// multiply pipe 62 % busy, 10.4 warp instructions per warp-butterfly (one column,
+// 2x: 63 %, 10.5).
 template <class F>
 struct TExpandCols {
   using X1 = TExpand<F, 8, false, true>;
