@@ -201,7 +201,8 @@ Status launch_tma_pass(sfntt_ctx* ctx, const TmaRequest& r, cudaStream_t s) {
   const uint32_t grid = std::min<uint32_t>(a.ntiles, ctas * (uint32_t)ctx->sm_count);
   launch_begin(ctx, s);
   // (LSTAGE: contiguous ranges of tiles per CTA, where an early launch gained nothing)
-  SFNTT_CU(launch_pdl(kern, grid, T::NT, smem, s, LSTAGE ? grid <= 16 : pdl_fits(grid, a.ntiles, a.log_n), min, mout, a));
+  const bool early = LSTAGE ? grid <= 16 : KD == Kind::S ? pdl_fits_strided(P, grid, a.ntiles, a.log_n) : pdl_fits(grid, a.ntiles, a.log_n);
+  SFNTT_CU(launch_pdl(kern, grid, T::NT, smem, s, early, min, mout, a));
   return launch_check(ctx, tma_pass_name<F, DESC, KD, P, PLAIN, TW, LSTAGE>(), s,
                       ((uint64_t)r.batch << log_w) * 8u);
 }
