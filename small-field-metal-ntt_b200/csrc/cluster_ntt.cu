@@ -314,8 +314,8 @@ uint32_t wide_clusters(const sfntt_ctx* ctx) {
 // x 15 10.0, 10.9, 8.3), but for the inverse of 2^16 points (x 10 6.9, 9.9, 9.0; x 15
 // 9.1, 11.8, 9.1).  Then 2^12 early again (2^15 x 36 9.7, 10.3, 10.9; inverse 9.3,
 // 11.6, 15.6).  2^13 points: only batches that 2^12 early suits come here.
-//   M31, whose twiddles come through L1: early up to 0.35 (2^16 x 3 5.0, 5.2, 7.3),
-// plainly up to 1.4 (2^14 x 24 7.7, 4.8, 6.7; 2^16 x 12 9.3, 7.5, 7.5), wide while
+//   M31, whose twiddles come through L1: early up to 0.24 (2^16 x 1 4.8, 5.2, 6.8),
+// plainly up to 1.4 (2^15 x 5 5.5, 4.9, 7.0; 2^14 x 24 7.7, 4.8, 6.7; 2^16 x 12 9.3, 7.5, 7.5), wide while
 // each has an SM (2^14 x 74 8.5, 8.6, 6.9), then early (2^15 x 37 9.0, 8.8, 13);
 // pairs that divide evenly early (2^13 x 148 6.0, 6.4, 6.7).
 // On several streams the forms differ by a tenth (8 streams, 2^14 x 55 4.0, 4.0,
@@ -332,7 +332,7 @@ ClusterForm cluster_form(const sfntt_ctx* ctx, uint32_t batch) {
     const bool wide = blocks <= 2 * sms && batch <= wide_clusters<F, DESC, X>(ctx);
     if (F::kMontgomery) return {wide && 25 * blocks > 19 * sms, !wide || 25 * blocks <= 19 * sms};
     if (X == 1 && blocks % sms == 0) return {false, true};
-    if (5 * blocks <= 7 * sms) return {false, 20 * blocks <= 7 * sms};
+    if (5 * blocks <= 7 * sms) return {false, 25 * blocks <= 6 * sms};
     return {wide, !wide};
   }
 }
