@@ -62,7 +62,7 @@ inline std::mutex mu;
 inline std::condition_variable cv;
 inline std::map<const void*, Mbar> mbars;
 inline std::vector<int> expired;                      // waits that ran out, per thread
-inline std::chrono::milliseconds limit{400};          // for every bounded wait
+inline std::chrono::milliseconds limit{1000};         // for every bounded wait
 inline int loads = 0, arrivals = 0;
 inline int lose_load = -1;                            // index of the load that never lands
 inline std::function<bool(uint32_t, int)> lose_arrival;  // (thread, index among all plain arrivals)
